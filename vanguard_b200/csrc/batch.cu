@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(BP) batch_step_kernel(BatchArgs a) {
             int c = ghost_index(s0 - 2 + slot, len, 0);
             double W[NW], U[NU];
             for (int v = 0; v < NW; v++) W[v] = a.in[v * a.plane + base + c];
-            M1::cons(W, q, U);
+            cons_of<M1>(W, q, U);
             for (int v = 0; v < NU; v++) Us[v][slot] = U[v];
         };
         conserve(p + 1);
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(BP) batch_step_kernel(BatchArgs a) {
                 u[v] = Us[v][p + 1];
                 uR[v] = Us[v][p + 2];
             }
-            evolve_edges<M1, 0>(uL, u, uR, kc, q, ub, ua, p >= 1, p <= BP - 2);
+            evolve_edges<M1, 0>(uL, u, uR, kc, q, ub, ua);
             for (int v = 0; v < NU; v++) Es[v][p] = ua[v];
         }
         __syncthreads();
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(BP) batch_step_kernel(BatchArgs a) {
         if (out_ok) {
             double Un[NU], W[NW];
             for (int v = 0; v < NU; v++) Un[v] = Us[v][p + 1] + (kc.r * (Fs[v][p] - Fs[v][p + 1]));
-            M1::setcons(Un, q, W);
+            setcons_of<M1>(Un, q, W);
             for (int v = 0; v < NW; v++) a.out[v * a.plane + base + cell] = W[v];
             if (bad_state<M1>(W, q)) atomicOr(a.err, ERR_STATE);
             double sw = M1::wave(W, q, 1);

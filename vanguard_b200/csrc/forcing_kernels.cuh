@@ -28,25 +28,25 @@ __device__ __forceinline__ int ghost1_index(int k, int n, int periodic) {
 // HPRSolvers::evolveStateByFractional{X,Y}TimeStep (Solvers/hprsolvers.cpp:606-620, :673-687) with
 // evolveStateByFractionalTimeStep (:791-797) on the conserved vectors of the three cells; the result is set into a
 // default-constructed state (primitive out).
-template <class M, int AXIS>
+template <class M, int AXIS, class D>
 __device__ __forceinline__ void frac_evolve_u(double frac, const double* uL, const double* uM, const double* uR,
                                               double dt, double dx, const SweepConst& k, const typename M::P& q,
-                                              double* out) {
+                                              double* out, D& dv) {
     constexpr int NU = M::NU;
-    double xl[NU], xr[NU], fl[NU], fr[NU];
+    double s[NU], xl[NU], xr[NU], fl[NU], fr[NU];
+    slopes_by<NU>(uL, uM, uR, k, s, dv);
 #pragma unroll
     for (int i = 0; i < NU; i++) {
-        double s = slope_f64(uL[i], uM[i], uR[i], k);
-        xl[i] = uM[i] - (0.5 * s);
-        xr[i] = uM[i] + (0.5 * s);
+        xl[i] = uM[i] - (0.5 * s[i]);
+        xr[i] = uM[i] + (0.5 * s[i]);
     }
-    M::template flux<AXIS>(xl, q, fl);
-    M::template flux<AXIS>(xr, q, fr);
+    flux_by<M, AXIS>(xl, q, fl, dv);
+    flux_by<M, AXIS>(xr, q, fr, dv);
     double c = frac * (dt / dx);
 #pragma unroll
     for (int i = 0; i < NU; i++) xl[i] = uM[i] + (c * (fl[i] - fr[i]));
     M::default_state(out);
-    M::setcons(xl, q, out);
+    setcons_by<M>(xl, q, out, dv);
 }
 
 // Neighbour round trip of every cell into a.aux (conserved planes): cons -> setConservedVariableVector on a
@@ -62,10 +62,10 @@ __global__ void __launch_bounds__(256) roundtrip_kernel(SweepArgs a) {
     const typename M::P q = M::params(a.params, a.ctrl ? a.ctrl->ch : a.ch_host);
     double W[NW], U[NU];
     for (int v = 0; v < NW; v++) W[v] = a.in[v * a.plane + self];
-    M::cons(W, q, U);
+    cons_of<M>(W, q, U);
     M::default_state(W);
-    M::setcons(U, q, W);
-    M::cons(W, q, U);
+    setcons_of<M>(U, q, W);
+    cons_of<M>(W, q, U);
     for (int v = 0; v < NU; v++) a.aux[v * a.plane + self] = U[v];
 }
 
@@ -83,19 +83,17 @@ struct forcing_blocks<M, decltype((void)M::FORCING_MIN_BLOCKS)> {
     static constexpr int value = M::FORCING_MIN_BLOCKS;
 };
 
-template <class M>
-__global__ void __launch_bounds__(FT, forcing_blocks<M>::value) forcing_kernel(SweepArgs a, int subcycles) {
+template <class M, class D>
+__device__ __forceinline__ void source_by(const double* U, const typename M::P& q, double* S, D& dv) {
+    if constexpr (shared_div<M>::value) M::source(U, q, S, dv);
+    else M::source(U, q, S);
+}
+
+// One cell's RK4 step into W; ksh holds k1, k2, k3 of the block's threads: [stage][component][thread].
+template <class M, class D>
+__device__ __forceinline__ void forcing_cell(const SweepArgs& a, int subcycles, int i, int j, double* ksh, double* W, D& dv) {
     constexpr int NU = M::NU, NW = M::NW;
-    extern __shared__ double ksh[];  // k1, k2, k3 of this block's threads: [stage][component][thread]
-    const long n = (long)a.nx * a.ny;
-    const long idx = blockIdx.x * (long)FT + threadIdx.x;
-    if (idx >= n) return;
-    const int i = (int)(idx / a.nx), j = (int)(idx - (long)i * a.nx);
     const long self = (long)i * a.pitch + j;
-    if (a.ctrl && !a.ctrl->active) {
-        for (int v = 0; v < NW; v++) a.out[v * a.plane + self] = a.in[v * a.plane + self];
-        return;
-    }
     // Solvers/hprsecondordersolver.cpp:516-519: time step 0.5 * (dt / subcyclingIterations)
     const double dt = 0.5 * ((a.ctrl ? a.ctrl->dt : a.dt_host) / subcycles);
     SweepConst k;
@@ -113,10 +111,10 @@ __global__ void __launch_bounds__(FT, forcing_blocks<M>::value) forcing_kernel(S
                         dims == 2 ? (long)ghost1_index(i - 1, a.ny, a.periodic) * a.pitch + j : self,
                         dims == 2 ? (long)ghost1_index(i + 1, a.ny, a.periodic) * a.pitch + j : self};
 
-    double uM[NU], S[NU], W[NW];
+    double uM[NU], S[NU];
     for (int v = 0; v < NW; v++) W[v] = a.in[v * a.plane + self];
-    M::cons(W, q, uM);
-    M::source(uM, q, S);
+    cons_by<M>(W, q, uM, dv);
+    source_by<M>(uM, q, S, dv);
     for (int v = 0; v < NU; v++) kk(0, v) = dt * S[v];
     const double stage_frac[3] = {0.5, 0.5, 1.0};
 #pragma unroll 1
@@ -124,7 +122,7 @@ __global__ void __launch_bounds__(FT, forcing_blocks<M>::value) forcing_kernel(S
         double ut[NU], wm[NW];
         for (int v = 0; v < NU; v++) ut[v] = uM[v] + (s < 2 ? (0.5 * kk(s, v)) : kk(s, v));
         M::default_state(wm);
-        M::setcons(ut, q, wm);
+        setcons_by<M>(ut, q, wm, dv);
         const double f = stage_frac[s];
         // dims == 1: X(f); dims == 2: X(f/2), Y(f), X(f/2)
         const int nsub = dims == 1 ? 1 : 3;
@@ -137,14 +135,14 @@ __global__ void __launch_bounds__(FT, forcing_blocks<M>::value) forcing_kernel(S
                 uA[v] = a.aux[v * a.plane + nb[2 * axis]];
                 uB[v] = a.aux[v * a.plane + nb[2 * axis + 1]];
             }
-            M::cons(wm, q, um);
+            cons_by<M>(wm, q, um, dv);
             if (axis == 0)
-                frac_evolve_u<M, 0>(fr, uA, um, uB, dt, a.dx, k, q, wm);
+                frac_evolve_u<M, 0>(fr, uA, um, uB, dt, a.dx, k, q, wm, dv);
             else
-                frac_evolve_u<M, 1>(fr, uA, um, uB, dt, a.dx, k, q, wm);
+                frac_evolve_u<M, 1>(fr, uA, um, uB, dt, a.dx, k, q, wm, dv);
         }
-        M::cons(wm, q, ut);
-        M::source(ut, q, S);
+        cons_by<M>(wm, q, ut, dv);
+        source_by<M>(ut, q, S, dv);
         if (s < 2)
             for (int v = 0; v < NU; v++) kk(s + 1, v) = dt * S[v];
     }
@@ -153,8 +151,45 @@ __global__ void __launch_bounds__(FT, forcing_blocks<M>::value) forcing_kernel(S
         const double k4 = dt * S[v];
         uM[v] = uM[v] + ((1.0 / 6.0) * (kk(0, v) + ((2.0 * kk(1, v)) + ((2.0 * kk(2, v)) + k4))));
     }
-    M::setcons(uM, q, W);  // the cell keeps its own primitives for fields setConservedVariableVector leaves alone
+    setcons_by<M>(uM, q, W, dv);  // the cell keeps its own primitives for fields setConservedVariableVector leaves alone
+}
+
+template <class M>
+__device__ __noinline__ void forcing_cell_ieee(const SweepArgs& a, int subcycles, int i, int j, double* ksh, double* W) {
+    IeeeDiv dv;
+    forcing_cell<M>(a, subcycles, i, j, ksh, W, dv);
+}
+
+template <class M>
+__global__ void __launch_bounds__(FT, forcing_blocks<M>::value) forcing_kernel(const __grid_constant__ SweepArgs a,
+                                                                               int subcycles) {
+    constexpr int NW = M::NW;
+    extern __shared__ double ksh[];
+    const long n = (long)a.nx * a.ny;
+    const long idx = blockIdx.x * (long)FT + threadIdx.x;
+    if (idx >= n) return;
+    const int i = (int)(idx / a.nx), j = (int)(idx - (long)i * a.nx);
+    const long self = (long)i * a.pitch + j;
+    if (a.ctrl && !a.ctrl->active) {
+        for (int v = 0; v < NW; v++) a.out[v * a.plane + self] = a.in[v * a.plane + self];
+        return;
+    }
+    double W[NW];
+    if constexpr (shared_div<M>::value) {
+        SharedDiv dv;
+        const bool shared = bias_shared(a.bias);
+        if (shared) forcing_cell<M>(a, subcycles, i, j, ksh, W, dv);
+        if (!shared || !dv.ok()) {  // an operand left the range of the shared reciprocals: the cell again with the compiler's division
+            double again[NW];
+            forcing_cell_ieee<M>(a, subcycles, i, j, ksh, again);
+            for (int v = 0; v < NW; v++) W[v] = again[v];
+        }
+    } else {
+        IeeeDiv dv;
+        forcing_cell<M>(a, subcycles, i, j, ksh, W, dv);
+    }
     for (int v = 0; v < NW; v++) a.out[v * a.plane + self] = W[v];
+    const typename M::P q = M::params(a.params, a.ctrl ? a.ctrl->ch : a.ch_host);
     if (bad_state<M>(W, q)) atomicOr(a.err, ERR_STATE);
 }
 

@@ -7,6 +7,7 @@
 // terms are exact additive zeros in every expression they appear in.
 #pragma once
 
+#include "exact_div.cuh"
 #include "vg_common.cuh"
 
 namespace vg {
@@ -19,6 +20,7 @@ struct EulerF64 {
     static constexpr int NW = NVEL + 2;
     static constexpr int NU = NW;
     static constexpr int IE = NU - 1;  // energy / pressure slot
+    static constexpr bool SHARED_DIV = true;
     static constexpr bool HAS_Y = NVEL == 2;
     static constexpr bool HAS_SOURCE = false;
     struct P {
@@ -27,7 +29,10 @@ struct EulerF64 {
     __device__ static P params(const double* prm, double /*ch*/) { return P{prm[0], prm[1], 0.0}; }
 
     // EulerEquationOfState::computeSpecificInternalEnergy (Euler/eulerequationofstate.cpp:7-13)
-    __device__ static double e_of(double rho, double p, const P& q) { return (p + (q.g * q.pinf)) / ((q.g - 1) * rho); }
+    template <class D>
+    __device__ static double e_of(double rho, double p, const P& q, D& dv) {
+        return dv.by((q.g - 1) * rho).positive(p + (q.g * q.pinf));
+    }
     // EulerEquationOfState::computePressure (Euler/eulerequationofstate.cpp:15-21)
     __device__ static double p_of(double rho, double e, const P& q) { return ((e * (q.g - 1)) * rho) - (q.g * q.pinf); }
 
@@ -37,33 +42,37 @@ struct EulerF64 {
     }
 
     // EulerStateVector::computeConservedVariableVector / computeTotalEnergy (Euler/eulerstatevector.cpp:78-91, :192-198)
-    __device__ static void cons(const double* W, const P& q, double* U) {
+    template <class D>
+    __device__ static void cons(const double* W, const P& q, double* U, D& dv) {
         double rho = W[0], u = W[1], v = (NVEL == 2) ? W[2] : 0.0, p = W[IE];
         U[0] = rho;
         U[1] = rho * u;
         if constexpr (NVEL == 2) U[2] = rho * v;
-        U[IE] = rho * ((0.5 * vsq(u, v)) + e_of(rho, p, q));
+        U[IE] = rho * ((0.5 * vsq(u, v)) + e_of(rho, p, q, dv));
     }
     // EulerStateVector::setConservedVariableVector (Euler/eulerstatevector.cpp:47-61)
-    __device__ static void setcons(const double* U, const P& q, double* W) {
+    template <class D>
+    __device__ static void setcons(const double* U, const P& q, double* W, D& dv) {
         double rho = U[0];
-        double u = U[1] / rho;
+        const auto by_rho = dv.by(rho);
+        double u = by_rho(U[1]);
         double v = 0.0;
-        if constexpr (NVEL == 2) v = U[2] / rho;
-        double e = (U[IE] / rho) - (0.5 * vsq(u, v));
+        if constexpr (NVEL == 2) v = by_rho(U[2]);
+        double e = by_rho.positive(U[IE]) - (0.5 * vsq(u, v));
         W[0] = rho;
         W[1] = u;
         if constexpr (NVEL == 2) W[2] = v;
         W[IE] = p_of(rho, e, q);
     }
     // EulerStateVector::compute{X,Y}FluxVector (Euler/eulerstatevector.cpp:93-120, :127-154)
-    template <int AXIS>
-    __device__ static void flux(const double* U, const P& q, double* F) {
+    template <int AXIS, class D>
+    __device__ static void flux(const double* U, const P& q, double* F, D& dv) {
         double rho = U[0];
-        double u = U[1] / rho;
+        const auto by_rho = dv.by(rho);
+        double u = by_rho(U[1]);
         double v = 0.0;
-        if constexpr (NVEL == 2) v = U[2] / rho;
-        double E = U[IE] / rho;
+        if constexpr (NVEL == 2) v = by_rho(U[2]);
+        double E = by_rho.positive(U[IE]);
         double e = E - (0.5 * vsq(u, v));
         double p = p_of(rho, e, q);
         if constexpr (AXIS == 0) {
@@ -91,6 +100,20 @@ struct EulerF64 {
         W[0] = 1.0;
         W[IE] = 1.0;
     }
+    // the same with the compiler's division
+    __device__ static void cons(const double* W, const P& q, double* U) {
+        IeeeDiv dv;
+        cons(W, q, U, dv);
+    }
+    __device__ static void setcons(const double* U, const P& q, double* W) {
+        IeeeDiv dv;
+        setcons(U, q, W, dv);
+    }
+    template <int AXIS>
+    __device__ static void flux(const double* U, const P& q, double* F) {
+        IeeeDiv dv;
+        flux<AXIS>(U, q, F, dv);
+    }
     __device__ static double density(const double* W) { return W[0]; }
     __device__ static double pressure(const double* W) { return W[IE]; }
 };
@@ -107,6 +130,7 @@ struct MHDF64 {
     static constexpr int IBX = IP + 1;
     static constexpr int IBY = IP + 2;
     static constexpr int IPSI = NW - 1;
+    static constexpr bool SHARED_DIV = true;
     static constexpr bool HAS_Y = true;
     static constexpr bool HAS_SOURCE = true;
     struct P {
@@ -117,6 +141,10 @@ struct MHDF64 {
     // MHDStateVector::computeSourceTermVector (MHD/mhdstatevector.cpp:222-234): GLM damping of psi with the
     // parabolic damping c_p = sqrt(c_h * 0.18) of MHDMaterialParameters::configureParabolicDamping
     // (MHD/mhdmaterialparameters.cpp:21-36), c_h being this step's maximum wave speed
+    template <class D>
+    __device__ static void source(const double* U, const P& q, double* S, D&) {
+        source(U, q, S);
+    }
     __device__ static void source(const double* U, const P& q, double* S) {
 #pragma unroll
         for (int i = 0; i < NU; i++) S[i] = 0.0;
@@ -124,7 +152,10 @@ struct MHDF64 {
         S[IPSI] = (-(q.ch2 / (cp * cp))) * U[IPSI];
     }
 
-    __device__ static double e_of(double rho, double p, const P& q) { return (p + (q.g * q.pinf)) / ((q.g - 1) * rho); }
+    template <class D>
+    __device__ static double e_of(double rho, double p, const P& q, D& dv) {
+        return dv.by((q.g - 1) * rho).positive(p + (q.g * q.pinf));
+    }
     __device__ static double p_of(double rho, double e, const P& q) { return ((e * (q.g - 1)) * rho) - (q.g * q.pinf); }
 
     __device__ static double sq3(double a, double b, double c) {
@@ -133,10 +164,11 @@ struct MHDF64 {
     }
 
     // MHDStateVector::computeConservedVariableVector + computeTotalEnergy (MHD/mhdstatevector.cpp:89-106, :236-245)
-    __device__ static void cons(const double* W, const P& q, double* U) {
+    template <class D>
+    __device__ static void cons(const double* W, const P& q, double* U, D& dv) {
         double rho = W[0], u = W[1], v = W[2], w = FULL ? W[3] : 0.0, p = W[IP];
         double bx = W[IBX], by = W[IBY], bz = FULL ? W[7] : 0.0;
-        double hydro = rho * ((0.5 * sq3(u, v, w)) + e_of(rho, p, q));
+        double hydro = rho * ((0.5 * sq3(u, v, w)) + e_of(rho, p, q, dv));
         U[0] = rho;
         U[1] = rho * u;
         U[2] = rho * v;
@@ -148,12 +180,14 @@ struct MHDF64 {
         U[IPSI] = W[IPSI];
     }
     // MHDStateVector::setConservedVariableVector (MHD/mhdstatevector.cpp:49-68)
-    __device__ static void setcons(const double* U, const P& q, double* W) {
+    template <class D>
+    __device__ static void setcons(const double* U, const P& q, double* W, D& dv) {
         double rho = U[0];
-        double u = U[1] / rho, v = U[2] / rho, w = 0.0;
-        if constexpr (FULL) w = U[3] / rho;
+        const auto by_rho = dv.by(rho);
+        double u = by_rho(U[1]), v = by_rho(U[2]), w = 0.0;
+        if constexpr (FULL) w = by_rho(U[3]);
         double bx = U[IBX], by = U[IBY], bz = FULL ? U[7] : 0.0;
-        double E = (U[IP] - (0.5 * sq3(bx, by, bz))) / rho;
+        double E = by_rho.positive(U[IP] - (0.5 * sq3(bx, by, bz)));
         double e = E - (0.5 * sq3(u, v, w));
         W[0] = rho;
         W[1] = u;
@@ -167,15 +201,16 @@ struct MHDF64 {
     }
     // MHDStateVector::compute{X,Y}FluxVector (MHD/mhdstatevector.cpp:108-158, :165-215); v.B is
     // VectorAlgebra::computeDotProduct summed from 0.0 (Mathematics/vectoralgebra.cpp:38-49).
-    template <int AXIS>
-    __device__ static void flux(const double* U, const P& q, double* F) {
+    template <int AXIS, class D>
+    __device__ static void flux(const double* U, const P& q, double* F, D& dv) {
         double rho = U[0];
-        double u = U[1] / rho, v = U[2] / rho, w = 0.0;
-        if constexpr (FULL) w = U[3] / rho;
+        const auto by_rho = dv.by(rho);
+        double u = by_rho(U[1]), v = by_rho(U[2]), w = 0.0;
+        if constexpr (FULL) w = by_rho(U[3]);
         double bx = U[IBX], by = U[IBY], bz = FULL ? U[7] : 0.0, psi = U[IPSI];
         double b2 = sq3(bx, by, bz);
         double E = U[IP];
-        double hydroE = (E - (0.5 * b2)) / rho;
+        double hydroE = by_rho.positive(E - (0.5 * b2));
         double e = hydroE - (0.5 * sq3(u, v, w));
         double p = p_of(rho, e, q);
         double vb = (0.0 + (u * bx)) + (v * by);
@@ -224,6 +259,20 @@ struct MHDF64 {
         W[0] = 1.0;
         W[IP] = 1.0;
     }
+    // the same with the compiler's division
+    __device__ static void cons(const double* W, const P& q, double* U) {
+        IeeeDiv dv;
+        cons(W, q, U, dv);
+    }
+    __device__ static void setcons(const double* U, const P& q, double* W) {
+        IeeeDiv dv;
+        setcons(U, q, W, dv);
+    }
+    template <int AXIS>
+    __device__ static void flux(const double* U, const P& q, double* F) {
+        IeeeDiv dv;
+        flux<AXIS>(U, q, F, dv);
+    }
     __device__ static double density(const double* W) { return W[0]; }
     __device__ static double pressure(const double* W) { return W[IP]; }
 };
@@ -237,6 +286,7 @@ struct MHDF64 {
 struct EulerReducedF64 {
     static constexpr int NW = 6;
     static constexpr int NU = 7;
+    static constexpr bool SHARED_DIV = true;
     static constexpr bool HAS_Y = true;
     static constexpr bool HAS_SOURCE = false;
     struct P {
@@ -251,12 +301,20 @@ struct EulerReducedF64 {
     }
     // EulerEquationOfState::computeSpecificInternalEnergy / computePressure / computeSoundSpeed
     // (Euler/eulerequationofstate.cpp:7-29) of material (g, pinf)
-    __device__ static double e_of(double rho, double p, double g, double pinf) { return (p + (g * pinf)) / ((g - 1) * rho); }
+    template <class D>
+    __device__ static double e_of(double rho, double p, double g, double pinf, D& dv) {
+        return dv.by((g - 1) * rho).positive(p + (g * pinf));
+    }
+    __device__ static double e_of(double rho, double p, double g, double pinf) {
+        IeeeDiv dv;
+        return e_of(rho, p, g, pinf, dv);
+    }
     __device__ static double p_of(double rho, double e, double g, double pinf) { return ((e * (g - 1)) * rho) - (g * pinf); }
     __device__ static double c_of(double rho, double p, double g, double pinf) { return sqrt((g * (p + pinf)) / rho); }
 
     // EulerReducedStateVector::computeConservedVariableVector (:96-129)
-    __device__ static void cons(const double* W, const P& q, double* U) {
+    template <class D>
+    __device__ static void cons(const double* W, const P& q, double* U, D& dv) {
         const double a1 = clamp_alpha(W[0]), a2 = 1.0 - a1;
         const double u = W[1], v = W[2], r1 = W[3], r2 = W[4], p = W[5];
         const double rho = (a1 * r1) + (a2 * r2);
@@ -267,30 +325,33 @@ struct EulerReducedF64 {
         U[4] = a1 * r1;
         U[5] = a2 * r2;
         const double v2 = (u * u) + (v * v);
-        const double E1 = e_of(rho, p, q.g1, q.pinf1) + (0.5 * v2), E2 = e_of(rho, p, q.g2, q.pinf2) + (0.5 * v2);
+        const double E1 = e_of(rho, p, q.g1, q.pinf1, dv) + (0.5 * v2), E2 = e_of(rho, p, q.g2, q.pinf2, dv) + (0.5 * v2);
         U[6] = rho * ((a1 * E1) + (a2 * E2));
     }
     // EulerReducedStateVector::setConservedVariableVector (:43-73)
-    __device__ static void setcons(const double* U, const P& q, double* W) {
+    template <class D>
+    __device__ static void setcons(const double* U, const P& q, double* W, D& dv) {
         const double rho = U[0];
-        const double a1 = clamp_alpha(U[1] / rho), a2 = 1.0 - a1;
-        const double u = U[2] / rho, v = U[3] / rho;
-        const double e = (U[6] / rho) - (0.5 * ((u * u) + (v * v)));
+        const auto by_rho = dv.by(rho);
+        const double a1 = clamp_alpha(by_rho.positive(U[1])), a2 = 1.0 - a1;
+        const double u = by_rho(U[2]), v = by_rho(U[3]);
+        const double e = by_rho.positive(U[6]) - (0.5 * ((u * u) + (v * v)));
         W[0] = a1;
         W[1] = u;
         W[2] = v;
-        W[3] = U[4] / a1;
-        W[4] = U[5] / a2;
+        W[3] = dv.by(a1).positive(U[4]);
+        W[4] = dv.by(a2).positive(U[5]);
         W[5] = (a1 * p_of(rho, e, q.g1, q.pinf1)) + (a2 * p_of(rho, e, q.g2, q.pinf2));
     }
     // EulerReducedStateVector::compute{X,Y}FluxVector(vector, params, params) (:131-180, :187-236)
-    template <int AXIS>
-    __device__ static void flux(const double* U, const P& q, double* F) {
+    template <int AXIS, class D>
+    __device__ static void flux(const double* U, const P& q, double* F, D& dv) {
         const double rho = U[0];
-        const double a1 = clamp_alpha(U[1] / rho), a2 = 1.0 - a1;
-        const double u = U[2] / rho, v = U[3] / rho;
-        const double r1 = U[4] / a1, r2 = U[5] / a2;
-        const double E = U[6] / rho;
+        const auto by_rho = dv.by(rho);
+        const double a1 = clamp_alpha(by_rho.positive(U[1])), a2 = 1.0 - a1;
+        const double u = by_rho(U[2]), v = by_rho(U[3]);
+        const double r1 = dv.by(a1).positive(U[4]), r2 = dv.by(a2).positive(U[5]);
+        const double E = by_rho.positive(U[6]);
         const double e = E - (0.5 * ((u * u) + (v * v)));
         const double p = (a1 * p_of(rho, e, q.g1, q.pinf1)) + (a2 * p_of(rho, e, q.g2, q.pinf2));
         const double un = AXIS == 0 ? u : v;
@@ -320,6 +381,20 @@ struct EulerReducedF64 {
         W[5] = 1.0;
     }
     // the smaller material density (bad-state check: both must stay positive) and the interface pressure
+    // the same with the compiler's division
+    __device__ static void cons(const double* W, const P& q, double* U) {
+        IeeeDiv dv;
+        cons(W, q, U, dv);
+    }
+    __device__ static void setcons(const double* U, const P& q, double* W) {
+        IeeeDiv dv;
+        setcons(U, q, W, dv);
+    }
+    template <int AXIS>
+    __device__ static void flux(const double* U, const P& q, double* F) {
+        IeeeDiv dv;
+        flux<AXIS>(U, q, F, dv);
+    }
     __device__ static double density(const double* W) { return W[3] < W[4] ? W[3] : W[4]; }
     __device__ static double pressure(const double* W) { return W[5]; }
 };
@@ -427,6 +502,7 @@ struct EulerMultiphysicsF64 {
 struct MHDReducedF64 {
     static constexpr int NW = 11;
     static constexpr int NU = 12;
+    static constexpr bool SHARED_DIV = true;
     static constexpr bool HAS_Y = true;
     static constexpr bool HAS_SOURCE = true;
     // GLM forcing at 8 resident blocks (128 registers): 7.6 % faster per 2048^2 step than at 6, same bits
@@ -445,7 +521,8 @@ struct MHDReducedF64 {
     __device__ static double b2_of(double bx, double by, double bz) { return ((bx * bx) + (by * by)) + (bz * bz); }
 
     // computeConservedVariableVector (:113-153)
-    __device__ static void cons(const double* W, const P& q, double* U) {
+    template <class D>
+    __device__ static void cons(const double* W, const P& q, double* U, D& dv) {
         const double a1 = R2::clamp_alpha(W[0]), a2 = 1.0 - a1;
         const double u = W[1], v = W[2], w = W[3], r1 = W[4], r2 = W[5], p = W[6], bx = W[7], by = W[8], bz = W[9];
         const double rho = (a1 * r1) + (a2 * r2);
@@ -458,8 +535,8 @@ struct MHDReducedF64 {
         U[6] = a2 * r2;
         const double v2 = ((u * u) + (v * v)) + (w * w);
         const double b2 = b2_of(bx, by, bz);
-        const double h1 = rho * ((0.5 * v2) + R2::e_of(rho, p, q.g1, q.pinf1));
-        const double h2 = rho * ((0.5 * v2) + R2::e_of(rho, p, q.g2, q.pinf2));
+        const double h1 = rho * ((0.5 * v2) + R2::e_of(rho, p, q.g1, q.pinf1, dv));
+        const double h2 = rho * ((0.5 * v2) + R2::e_of(rho, p, q.g2, q.pinf2, dv));
         U[7] = (a1 * (h1 + (0.5 * b2))) + (a2 * (h2 + (0.5 * b2)));
         U[8] = bx;
         U[9] = by;
@@ -467,19 +544,21 @@ struct MHDReducedF64 {
         U[11] = W[10];
     }
     // setConservedVariableVector (:58-89)
-    __device__ static void setcons(const double* U, const P& q, double* W) {
+    template <class D>
+    __device__ static void setcons(const double* U, const P& q, double* W, D& dv) {
         const double rho = U[0];
-        const double a1 = R2::clamp_alpha(U[1] / rho), a2 = 1.0 - a1;
-        const double u = U[2] / rho, v = U[3] / rho, w = U[4] / rho;
+        const auto by_rho = dv.by(rho);
+        const double a1 = R2::clamp_alpha(by_rho.positive(U[1])), a2 = 1.0 - a1;
+        const double u = by_rho(U[2]), v = by_rho(U[3]), w = by_rho(U[4]);
         const double bx = U[8], by = U[9], bz = U[10];
-        const double E = (U[7] - (0.5 * b2_of(bx, by, bz))) / rho;
+        const double E = by_rho.positive(U[7] - (0.5 * b2_of(bx, by, bz)));
         const double e = E - (0.5 * (((u * u) + (v * v)) + (w * w)));
         W[0] = a1;
         W[1] = u;
         W[2] = v;
         W[3] = w;
-        W[4] = U[5] / a1;
-        W[5] = U[6] / a2;
+        W[4] = dv.by(a1).positive(U[5]);
+        W[5] = dv.by(a2).positive(U[6]);
         W[6] = (a1 * R2::p_of(rho, e, q.g1, q.pinf1)) + (a2 * R2::p_of(rho, e, q.g2, q.pinf2));
         W[7] = bx;
         W[8] = by;
@@ -488,17 +567,18 @@ struct MHDReducedF64 {
     }
     // compute{X,Y}FluxVector(vector, params, params) (:155-232, :239-316); v.B summed from 0.0 as
     // VectorAlgebra::computeDotProduct (Mathematics/vectoralgebra.cpp:38-49)
-    template <int AXIS>
-    __device__ static void flux(const double* U, const P& q, double* F) {
+    template <int AXIS, class D>
+    __device__ static void flux(const double* U, const P& q, double* F, D& dv) {
         const double rho = U[0];
-        const double a1 = R2::clamp_alpha(U[1] / rho), a2 = 1.0 - a1;
-        const double u = U[2] / rho, v = U[3] / rho, w = U[4] / rho;
-        const double r1 = U[5] / a1, r2 = U[6] / a2;
+        const auto by_rho = dv.by(rho);
+        const double a1 = R2::clamp_alpha(by_rho.positive(U[1])), a2 = 1.0 - a1;
+        const double u = by_rho(U[2]), v = by_rho(U[3]), w = by_rho(U[4]);
+        const double r1 = dv.by(a1).positive(U[5]), r2 = dv.by(a2).positive(U[6]);
         const double bx = U[8], by = U[9], bz = U[10], psi = U[11];
         const double v2 = ((u * u) + (v * v)) + (w * w);
         const double b2 = b2_of(bx, by, bz);
         const double E = U[7];
-        const double e = ((E - (0.5 * b2)) / rho) - (0.5 * v2);
+        const double e = by_rho.positive(E - (0.5 * b2)) - (0.5 * v2);
         const double p = (a1 * R2::p_of(rho, e, q.g1, q.pinf1)) + (a2 * R2::p_of(rho, e, q.g2, q.pinf2));
         const double ch2 = (a1 * q.ch2) + (a2 * q.ch2);
         const double vb = ((0.0 + (u * bx)) + (v * by)) + (w * bz);
@@ -527,12 +607,13 @@ struct MHDReducedF64 {
         F[11] = ch2 * bn;
     }
     // computeSourceTermVector (:323-347): GLM damping of psi
-    __device__ static void source(const double* U, const P& q, double* S) {
+    template <class D>
+    __device__ static void source(const double* U, const P& q, double* S, D& dv) {
 #pragma unroll
         for (int i = 0; i < NU; i++) S[i] = 0.0;
-        const double a1 = R2::clamp_alpha(U[1] / U[0]), a2 = 1.0 - a1;
+        const double a1 = R2::clamp_alpha(dv.by(U[0]).positive(U[1])), a2 = 1.0 - a1;
         const double ch2 = (a1 * q.ch2) + (a2 * q.ch2), cp2 = (a1 * q.cp2) + (a2 * q.cp2);
-        S[11] = (-(ch2 / cp2)) * U[11];
+        S[11] = (-dv.by(cp2).positive(ch2)) * U[11];
     }
     // MHDWaveSpeeds::compute{X,Y}FastMagnetoAcousticSpeed (MHD/mhdwavespeeds.cpp:7-17, :43-63) of material (g, pinf)
     // at density rho and normal field bn; the Alfven speed is computeNorm(B) / sqrt(rho), the norm summed from 0.0
@@ -564,6 +645,24 @@ struct MHDReducedF64 {
         W[6] = 1.0;
     }
     // the smaller material density (bad-state check) and the interface pressure
+    // the same with the compiler's division
+    __device__ static void cons(const double* W, const P& q, double* U) {
+        IeeeDiv dv;
+        cons(W, q, U, dv);
+    }
+    __device__ static void setcons(const double* U, const P& q, double* W) {
+        IeeeDiv dv;
+        setcons(U, q, W, dv);
+    }
+    template <int AXIS>
+    __device__ static void flux(const double* U, const P& q, double* F) {
+        IeeeDiv dv;
+        flux<AXIS>(U, q, F, dv);
+    }
+    __device__ static void source(const double* U, const P& q, double* S) {
+        IeeeDiv dv;
+        source(U, q, S, dv);
+    }
     __device__ static double density(const double* W) { return W[4] < W[5] ? W[4] : W[5]; }
     __device__ static double pressure(const double* W) { return W[6]; }
 };

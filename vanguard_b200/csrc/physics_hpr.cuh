@@ -19,6 +19,7 @@
 //           sigma0, n}
 #pragma once
 
+#include "exact_div.cuh"
 #include "vg_common.cuh"
 
 namespace vg {
@@ -30,6 +31,7 @@ template <bool SOLID>
 struct HPRModel {
     static constexpr int NW = 17;
     static constexpr int NU = 17;
+    static constexpr bool SHARED_DIV = !SOLID;  // the solid equations of state divide as the compiler does
     static constexpr bool HAS_Y = true;
     static constexpr bool HAS_SOURCE = true;
     static constexpr int J_PLANE = 14;  // first heat-flux plane (kept by setConservedVariableVector when cold)
@@ -76,14 +78,19 @@ struct HPRModel {
         return r;
     }
     // TensorAlgebra::computeDeviator (Mathematics/tensoralgebra.cpp:27-30)
-    __device__ static M3 dev(const M3& g) {
-        double c = (((0.0 + g.m[0][0]) + g.m[1][1]) + g.m[2][2]) / 3.0;
+    template <class D>
+    __device__ static M3 dev(const M3& g, D& dv) {
+        double c = dv.third(((0.0 + g.m[0][0]) + g.m[1][1]) + g.m[2][2]);
         M3 r;
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
             for (int j = 0; j < 3; j++) r.m[i][j] = g.m[i][j] + (-1.0 * (c * (i == j ? 1.0 : 0.0)));
         return r;
+    }
+    __device__ static M3 dev(const M3& g) {
+        IeeeDiv dv;
+        return dev(g, dv);
     }
     __device__ static double det(const M3& a) {  // Mathematics/matrixalgebra.cpp:131-135
         return ((a.m[0][0] * ((a.m[1][1] * a.m[2][2]) - (a.m[2][1] * a.m[1][2]))) -
@@ -114,7 +121,12 @@ struct HPRModel {
         return -q.pinf;
     }
     __device__ static double mg_eref(double rho, const P& q) {  // computeReferenceInternalEnergy (:68-102)
-        if constexpr (!SOLID) return q.pinf / rho;
+        IeeeDiv dv;
+        return mg_eref(rho, q, dv.by(rho));
+    }
+    template <class By>
+    __device__ static double mg_eref(double rho, const P& q, const By& by_rho) {
+        if constexpr (!SOLID) return by_rho(q.pinf);
         if (q.eos == 1) return rho > q.rho0 ? (0.5 * q.pref_mat) * ((1.0 / q.rho0) - (1.0 / rho)) : 0.0;
         if (q.eos == 2) {
             double c = gr_coef(rho, q);
@@ -152,14 +164,21 @@ struct HPRModel {
         return -(q.pinf / (rho * rho));
     }
     // computeInternalEnergy / computePressure / computeTemperature (:194-221)
-    __device__ static double mg_energy(double rho, double p, const P& q) {
-        return mg_eref(rho, q) + ((p - mg_pref(rho, q)) / (rho * mg_G(rho, q)));
+    template <class D>
+    __device__ static double mg_energy(double rho, double p, const P& q, D& dv) {
+        return mg_eref(rho, q, dv.by(rho)) + dv.by(rho * mg_G(rho, q)).positive(p - mg_pref(rho, q));
     }
-    __device__ static double mg_pressure(double rho, double e, const P& q) {
-        return (((e - mg_eref(rho, q)) * rho) * mg_G(rho, q)) + mg_pref(rho, q);
+    template <class By>
+    __device__ static double mg_pressure(double rho, double e, const P& q, const By& by_rho) {
+        return (((e - mg_eref(rho, q, by_rho)) * rho) * mg_G(rho, q)) + mg_pref(rho, q);
+    }
+    template <class D>
+    __device__ static double mg_temperature(double rho, double p, const P& q, D& dv) {
+        return q.Tref + dv.by((rho * mg_G(rho, q)) * q.cv).positive(p - mg_pref(rho, q));
     }
     __device__ static double mg_temperature(double rho, double p, const P& q) {
-        return q.Tref + ((p - mg_pref(rho, q)) / ((rho * mg_G(rho, q)) * q.cv));
+        IeeeDiv dv;
+        return mg_temperature(rho, p, q, dv);
     }
     // computeInternalEnergyDerivativeDensity / Pressure, computeTemperatureDerivativeDensity / Pressure (:223-262)
     __device__ static double mg_dedrho(double rho, double p, const P& q) {
@@ -174,8 +193,9 @@ struct HPRModel {
     __device__ static double mg_dTdp(double rho, const P& q) { return mg_dedp(rho, q) / q.cv; }
 
     // ---- HPREquationOfState (HPR/hprequationofstate.cpp:7-81)
-    __device__ static double meso_distortion(const M3& A, const P& q) {
-        M3 D = dev(tmul(A, A));
+    template <class Dv>
+    __device__ static double meso_distortion(const M3& A, const P& q, Dv& dv) {
+        M3 D = dev(tmul(A, A), dv);
         double sum = 0.0;
 #pragma unroll
         for (int i = 0; i < 3; i++) sum += ((0.0 + (D.m[i][0] * D.m[i][0])) + (D.m[i][1] * D.m[i][1])) + (D.m[i][2] * D.m[i][2]);
@@ -185,21 +205,38 @@ struct HPRModel {
         return (0.5 * (q.alpha * q.alpha)) * (((jx * jx) + (jy * jy)) + (jz * jz));
     }
     __device__ static double macro(double u, double v, double w) { return 0.5 * (((u * u) + (v * v)) + (w * w)); }
+    template <class D>
     __device__ static double total_energy(double rho, double p, double u, double v, double w, const M3& A, double jx, double jy,
-                                          double jz, const P& q) {
-        double E = (mg_energy(rho, p, q) + meso_distortion(A, q)) + macro(u, v, w);
+                                          double jz, const P& q, D& dv) {
+        double E = (mg_energy(rho, p, q, dv) + meso_distortion(A, q, dv)) + macro(u, v, w);
         if (q.thermal) E += meso_thermal(jx, jy, jz, q);
         return E;
     }
+    __device__ static double total_energy(double rho, double p, double u, double v, double w, const M3& A, double jx, double jy,
+                                          double jz, const P& q) {
+        IeeeDiv dv;
+        return total_energy(rho, p, u, v, w, A, jx, jy, jz, q, dv);
+    }
+    template <class By, class D>
+    __device__ static double pressure_of(double rho, double E, double u, double v, double w, const M3& A, double jx, double jy,
+                                         double jz, const P& q, const By& by_rho, D& dv) {
+        double e = E - (macro(u, v, w) + meso_distortion(A, q, dv));
+        if (q.thermal) e -= meso_thermal(jx, jy, jz, q);
+        return mg_pressure(rho, e, q, by_rho);
+    }
     __device__ static double pressure_of(double rho, double E, double u, double v, double w, const M3& A, double jx, double jy,
                                          double jz, const P& q) {
-        double e = E - (macro(u, v, w) + meso_distortion(A, q));
-        if (q.thermal) e -= meso_thermal(jx, jy, jz, q);
-        return mg_pressure(rho, e, q);
+        IeeeDiv dv;
+        return pressure_of(rho, E, u, v, w, A, jx, jy, jz, q, dv.by(rho), dv);
     }
     // c_s^2 A dev(A^T A)   (HPR/hprderivatives.cpp:17-25)
     __device__ static M3 dEdA(const M3& A, const P& q) {
-        M3 AD = mul(A, dev(tmul(A, A)));
+        IeeeDiv dv;
+        return dEdA(A, q, dv);
+    }
+    template <class D>
+    __device__ static M3 dEdA(const M3& A, const P& q, D& dv) {
+        M3 AD = mul(A, dev(tmul(A, A), dv));
         double cs2 = q.cs * q.cs;
         M3 r;
 #pragma unroll
@@ -210,11 +247,12 @@ struct HPRModel {
     }
 
     // HPRStateVector::computeConservedVariableVector (HPR/hprstatevector.cpp:134-162)
-    __device__ static void cons(const double* W, const P& q, double* U) {
+    template <class D>
+    __device__ static void cons(const double* W, const P& q, double* U, D& dv) {
         M3 A = load(W + 2);
         double rho = W[0];
         U[0] = rho;
-        U[1] = rho * total_energy(rho, W[1], W[11], W[12], W[13], A, W[14], W[15], W[16], q);
+        U[1] = rho * total_energy(rho, W[1], W[11], W[12], W[13], A, W[14], W[15], W[16], q, dv);
 #pragma unroll
         for (int i = 0; i < 9; i++) U[2 + i] = W[2 + i];
         U[11] = rho * W[11];
@@ -225,36 +263,39 @@ struct HPRModel {
         U[16] = q.thermal ? rho * W[16] : 0.0;
     }
     // HPRStateVector::setConservedVariableVector (HPR/hprstatevector.cpp:78-103); J kept when not thermal
-    __device__ static void setcons(const double* U, const P& q, double* W) {
+    template <class D>
+    __device__ static void setcons(const double* U, const P& q, double* W, D& dv) {
         double rho = U[0];
+        const auto by_rho = dv.by(rho);
         W[0] = rho;
 #pragma unroll
         for (int i = 0; i < 9; i++) W[2 + i] = U[2 + i];
-        W[11] = U[11] / rho;
-        W[12] = U[12] / rho;
-        W[13] = U[13] / rho;
+        W[11] = by_rho(U[11]);
+        W[12] = by_rho(U[12]);
+        W[13] = by_rho(U[13]);
         if (q.thermal) {
-            W[14] = U[14] / rho;
-            W[15] = U[15] / rho;
-            W[16] = U[16] / rho;
+            W[14] = by_rho(U[14]);
+            W[15] = by_rho(U[15]);
+            W[16] = by_rho(U[16]);
         }
         M3 A = load(W + 2);
-        W[1] = pressure_of(rho, U[1] / rho, W[11], W[12], W[13], A, W[14], W[15], W[16], q);
+        W[1] = pressure_of(rho, by_rho.positive(U[1]), W[11], W[12], W[13], A, W[14], W[15], W[16], q, by_rho, dv);
     }
     // HPRStateVector::compute{X,Y}FluxVector (HPR/hprstatevector.cpp:164-298)
-    template <int AXIS>
-    __device__ static void flux(const double* U, const P& q, double* F) {
+    template <int AXIS, class D>
+    __device__ static void flux(const double* U, const P& q, double* F, D& dv) {
         double rho = U[0];
+        const auto by_rho = dv.by(rho);
         M3 A = load(U + 2);
-        M3 d = dEdA(A, q);
+        M3 d = dEdA(A, q, dv);
         M3 Pm = tmul(A, d);
         double sig[3];
 #pragma unroll
         for (int i = 0; i < 3; i++) sig[i] = (-rho) * Pm.m[AXIS][i];
-        double u = U[11] / rho, v = U[12] / rho, w = U[13] / rho;
-        double jx = U[14] / rho, jy = U[15] / rho, jz = U[16] / rho;
-        double E = U[1] / rho;
-        double p = pressure_of(rho, E, u, v, w, A, jx, jy, jz, q);
+        double u = by_rho(U[11]), v = by_rho(U[12]), w = by_rho(U[13]);
+        double jx = by_rho(U[14]), jy = by_rho(U[15]), jz = by_rho(U[16]);
+        double E = by_rho.positive(U[1]);
+        double p = pressure_of(rho, E, u, v, w, A, jx, jy, jz, q, by_rho, dv);
         double un = AXIS == 0 ? u : v;
 #pragma unroll
         for (int i = 0; i < 17; i++) F[i] = 0.0;
@@ -275,7 +316,7 @@ struct HPRModel {
 #pragma unroll
         for (int i = 0; i < 3; i++) F[2 + (i * 3) + AXIS] = ((0.0 + (A.m[i][0] * u)) + (A.m[i][1] * v)) + (A.m[i][2] * w);
         if (q.thermal) {
-            double T = mg_temperature(rho, p, q);
+            double T = mg_temperature(rho, p, q, dv);
             double a2 = q.alpha * q.alpha;
             F[1] += T * (a2 * (AXIS == 0 ? jx : jy));
             if (AXIS == 0) {
@@ -293,8 +334,13 @@ struct HPRModel {
     // scales it by (min(|sigma|, 1e8) / sigma0)^n, |sigma| = TensorAlgebra::computeSigmaNorm
     // (Mathematics/tensoralgebra.cpp:276-283) of sigma = -rho A^T dE/dA, with std::min's tie rule
     __device__ static double theta1(double rho, const M3& A, const M3& d, const P& q) {
+        IeeeDiv dv;
+        return theta1(rho, A, d, q, dv);
+    }
+    template <class D>
+    __device__ static double theta1(double rho, const M3& A, const M3& d, const P& q, D& dv) {
         const double cs2 = q.cs * q.cs;
-        const double th = 3.0 * (pow(det(A), (5.0 / 3.0)) / (cs2 * q.tau1));
+        const double th = 3.0 * dv.by(cs2 * q.tau1).positive(pow(det(A), (5.0 / 3.0)));
         if (!SOLID || !q.plastic) return th;
         M3 Pm = tmul(A, d);
         double t[3][3];
@@ -311,11 +357,12 @@ struct HPRModel {
         return th * pow(nrm / q.sigma0, q.npl);
     }
     // HPRStateVector::computeSourceTermVector (HPR/hprstatevector.cpp:312-366), HPRSourceTerms (HPR/hprsourceterms.cpp:7-39)
-    __device__ static void source(const double* U, const P& q, double* S) {
+    template <class D>
+    __device__ static void source(const double* U, const P& q, double* S, D& dv) {
         double rho = U[0];
         M3 A = load(U + 2);
-        M3 d = dEdA(A, q);
-        double th1 = theta1(rho, A, d, q);
+        M3 d = dEdA(A, q, dv);
+        double th1 = theta1(rho, A, d, q, dv);
 #pragma unroll
         for (int i = 0; i < 17; i++) S[i] = 0.0;
 #pragma unroll
@@ -323,17 +370,37 @@ struct HPRModel {
 #pragma unroll
             for (int j = 0; j < 3; j++) S[2 + (i * 3) + j] = -d.m[i][j] * th1;
         if (q.thermal) {
-            double E = U[1] / rho;
-            double u = U[11] / rho, v = U[12] / rho, w = U[13] / rho;
-            double jx = U[14] / rho, jy = U[15] / rho, jz = U[16] / rho;
-            double p = pressure_of(rho, E, u, v, w, A, jx, jy, jz, q);
-            double T = mg_temperature(rho, p, q);
+            const auto by_rho = dv.by(rho);
+            double E = by_rho.positive(U[1]);
+            double u = by_rho(U[11]), v = by_rho(U[12]), w = by_rho(U[13]);
+            double jx = by_rho(U[14]), jy = by_rho(U[15]), jz = by_rho(U[16]);
+            double p = pressure_of(rho, E, u, v, w, A, jx, jy, jz, q, by_rho, dv);
+            double T = mg_temperature(rho, p, q, dv);
             double a2 = q.alpha * q.alpha;
-            double th2 = 1.0 / ((a2 * q.tau2) * ((rho / q.rho0) * (q.T0 / T)));
+            double th2 = dv.by((a2 * q.tau2) * (dv.by(q.rho0).positive(rho) * dv.by(T).positive(q.T0))).positive(1.0);
             S[14] = ((-rho) * th2) * (a2 * jx);
             S[15] = ((-rho) * th2) * (a2 * jy);
             S[16] = ((-rho) * th2) * (a2 * jz);
         }
+    }
+
+    // the same with the compiler's division
+    __device__ static void cons(const double* W, const P& q, double* U) {
+        IeeeDiv dv;
+        cons(W, q, U, dv);
+    }
+    __device__ static void setcons(const double* U, const P& q, double* W) {
+        IeeeDiv dv;
+        setcons(U, q, W, dv);
+    }
+    template <int AXIS>
+    __device__ static void flux(const double* U, const P& q, double* F) {
+        IeeeDiv dv;
+        flux<AXIS>(U, q, F, dv);
+    }
+    __device__ static void source(const double* U, const P& q, double* S) {
+        IeeeDiv dv;
+        source(U, q, S, dv);
     }
 
     // HPRAcousticTensor::computeMaximumWaveSpeed (HPR/hpracoustictensor.cpp:7-97) with the 10-step power iteration of

@@ -13,11 +13,39 @@
 // sliding window of the stencil in registers; a warp reads 32 consecutive doubles per plane-row.
 #pragma once
 
+#include <type_traits>
 #include <utility>
 
+#include "exact_div.cuh"
 #include "vg_common.cuh"
 
 namespace vg {
+
+// Models whose conversions and fluxes are templates over a division policy (exact_div.cuh) name SHARED_DIV; the others
+// divide as the compiler does.
+template <class M, class = void>
+struct shared_div {
+    static constexpr bool value = false;
+};
+template <class M>
+struct shared_div<M, decltype((void)M::SHARED_DIV)> {
+    static constexpr bool value = M::SHARED_DIV;
+};
+template <class M, class D>
+__device__ __forceinline__ void cons_by(const double* W, const typename M::P& q, double* U, D& dv) {
+    if constexpr (shared_div<M>::value) M::cons(W, q, U, dv);
+    else M::cons(W, q, U);
+}
+template <class M, class D>
+__device__ __forceinline__ void setcons_by(const double* U, const typename M::P& q, double* W, D& dv) {
+    if constexpr (shared_div<M>::value) M::setcons(U, q, W, dv);
+    else M::setcons(U, q, W);
+}
+template <class M, int AXIS, class D>
+__device__ __forceinline__ void flux_by(const double* U, const typename M::P& q, double* F, D& dv) {
+    if constexpr (shared_div<M>::value) M::template flux<AXIS>(U, q, F, dv);
+    else M::template flux<AXIS>(U, q, F);
+}
 
 // SlopeLimiters::computeSlopeLimiter (Solvers/slopelimiters.cpp:7-74)
 __device__ __forceinline__ double limiter_f64(double r, double w, int id) {
@@ -35,34 +63,73 @@ __device__ __forceinline__ double limiter_f64(double r, double w, int id) {
     return std_min(1.0, 2.0 / ((1.0 - w) + ((1.0 + w) * r)));
 }
 
-// One component of SlopeLimiters::computeSlopeVector (Solvers/slopelimiters.cpp:217-246).
-__device__ __forceinline__ double slope_f64(double uL, double u, double uR, const SweepConst& k) {
-    double dm = u - uL;
-    double dp = uR - u;
-    double s = (k.cm * dm) + (k.cp * dp);
-    double num = dm, den = dp;
-    if (fabs(num) < k.floor5) num = k.floor5;
-    if (fabs(den) < k.floor5) den = k.floor5;
-    return s * limiter_f64(num / den, k.bias, k.limiter);
+// The same without branches for |w| <= 1 and a ratio r of nonzero numbers of magnitudes in [1e-5, 2^513): every quotient
+// is formed, and the ones that the reference's branch does not reach are not used.  r is compared with 0, 1/2 and 1 by
+// its upper word (the constants' lower words are zero).  For r >= 1 the second divisor is at least 2 to within a
+// rounding, so xi_R stays below 2 and the reference's outer minimum with 2 cannot bite.
+template <int ID>
+__device__ __forceinline__ double limiter_shared(double r, double w) {
+    const int hi = __double2hiint(r);
+    const bool low = hi < 0x3ff00000;
+    const double xi = SharedDiv::known(2.0, (1.0 - w) + ((1.0 + w) * r));
+    double phi;
+    if constexpr (ID == 0)
+        phi = low ? (hi < 0x3fe00000 ? 2.0 * r : 1.0) : std_min(r, xi);
+    else if constexpr (ID == 1)
+        phi = std_min(SharedDiv::known(2.0 * r, 1.0 + r), xi);
+    else
+        phi = low ? r : std_min(1.0, xi);
+    return hi < 0 ? 0.0 : phi;
 }
+
+// SlopeLimiters::computeSlopeVector (Solvers/slopelimiters.cpp:217-246) of n components.  The limiter is chosen outside
+// the loop, so that the components' chains of divisions overlap.
+template <int ID, int N, class D>
+__device__ __forceinline__ void slopes_of(const double* uL, const double* u, const double* uR, const SweepConst& k,
+                                          double* s, D& dv) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const double dm = u[i] - uL[i], dp = uR[i] - u[i];
+        double num = dm, den = dp;
+        if (fabs(num) < k.floor5) num = k.floor5;
+        if (fabs(den) < k.floor5) den = k.floor5;
+        double phi;
+        if constexpr (std::is_same<D, SharedDiv>::value) {
+            dv.note_below(dm);
+            dv.note_below(dp);
+            phi = limiter_shared<ID>(SharedDiv::known(num, den), k.bias);
+        } else {
+            phi = limiter_f64(num / den, k.bias, ID);
+        }
+        s[i] = ((k.cm * dm) + (k.cp * dp)) * phi;
+    }
+}
+template <int N, class D>
+__device__ __forceinline__ void slopes_by(const double* uL, const double* u, const double* uR, const SweepConst& k,
+                                          double* s, D& dv) {
+    if (k.limiter == 0) slopes_of<0, N>(uL, u, uR, k, s, dv);
+    else if (k.limiter == 1) slopes_of<1, N>(uL, u, uR, k, s, dv);
+    else slopes_of<2, N>(uL, u, uR, k, s, dv);
+}
+// whether the branch-free limiter covers this bias
+__device__ __forceinline__ bool bias_shared(double w) { return fabs(w) <= 1.0; }
 
 // Solvers::evolveStateByHalf{X,Y}TimeStep for both sides of one cell (Solvers/solvers.cpp:454-466,
 // :502-514, :550-565): returns the conserved vectors of the two evolved edge states after the reference's
 // primitive round trip (setConservedVariableVector then computeConservedVariableVector).
-template <class M, int AXIS>
-__device__ __forceinline__ void evolve_edges(const double* uL, const double* u, const double* uR, const SweepConst& k,
-                                             const typename M::P& q, double* ua_left_side, double* ua_right_side,
-                                             bool want_left, bool want_right) {
+template <class M, int AXIS, class D>
+__device__ __forceinline__ void evolve_edges_by(const double* uL, const double* u, const double* uR, const SweepConst& k,
+                                                const typename M::P& q, double* ua_left_side, double* ua_right_side, D& dv) {
     constexpr int NU = M::NU;
-    double xl[NU], xr[NU], fl[NU], fr[NU];
+    double s[NU], xl[NU], xr[NU], fl[NU], fr[NU];
+    slopes_by<NU>(uL, u, uR, k, s, dv);
 #pragma unroll
     for (int i = 0; i < NU; i++) {
-        double s = slope_f64(uL[i], u[i], uR[i], k);
-        xl[i] = u[i] - (0.5 * s);
-        xr[i] = u[i] + (0.5 * s);
+        xl[i] = u[i] - (0.5 * s[i]);
+        xr[i] = u[i] + (0.5 * s[i]);
     }
-    M::template flux<AXIS>(xl, q, fl);
-    M::template flux<AXIS>(xr, q, fr);
+    flux_by<M, AXIS>(xl, q, fl, dv);
+    flux_by<M, AXIS>(xr, q, fr, dv);
     double a[NU], b[NU];
 #pragma unroll
     for (int i = 0; i < NU; i++) {
@@ -71,32 +138,149 @@ __device__ __forceinline__ void evolve_edges(const double* uL, const double* u, 
         b[i] = xr[i] + ev;
     }
     double w[M::NW];
-    if (want_left) {
-        M::setcons(a, q, w);
-        M::cons(w, q, ua_left_side);
-    }
-    if (want_right) {
-        M::setcons(b, q, w);
-        M::cons(w, q, ua_right_side);
-    }
+    setcons_by<M>(a, q, w, dv);
+    cons_by<M>(w, q, ua_left_side, dv);
+    setcons_by<M>(b, q, w, dv);
+    cons_by<M>(w, q, ua_right_side, dv);
 }
 
 // FirstOrderSolver::compute{X,Y}FORCEFlux (Solvers/firstordersolver.cpp:173-230) on the conserved vectors
 // of the left state ua and right state ub.
-template <class M, int AXIS>
-__device__ __forceinline__ void force_flux(const double* ua, const double* ub, const SweepConst& k,
-                                           const typename M::P& q, double* F) {
+template <class M, int AXIS, class D>
+__device__ __forceinline__ void force_flux_by(const double* ua, const double* ub, const SweepConst& k,
+                                              const typename M::P& q, double* F, D& dv) {
     constexpr int NU = M::NU;
     double fa[NU], fb[NU], uri[NU], fri[NU];
-    M::template flux<AXIS>(ua, q, fa);
-    M::template flux<AXIS>(ub, q, fb);
+    flux_by<M, AXIS>(ua, q, fa, dv);
+    flux_by<M, AXIS>(ub, q, fb, dv);
 #pragma unroll
     for (int i = 0; i < NU; i++) uri[i] = 0.5 * ((ua[i] + ub[i]) + (k.r * (fa[i] - fb[i])));
-    M::template flux<AXIS>(uri, q, fri);
+    flux_by<M, AXIS>(uri, q, fri, dv);
 #pragma unroll
     for (int i = 0; i < NU; i++) {
         double lf = 0.5 * ((fa[i] + fb[i]) + (k.rinv * (ua[i] - ub[i])));
         F[i] = 0.5 * (lf + fri[i]);
+    }
+}
+
+// The stages of a sweep as its kernels call them: the shared-reciprocal form, and again with the compiler's division
+// where an operand left the proven range (a call out of line, so that the common path holds no second copy of it).
+template <class M, int AXIS>
+__device__ __noinline__ void evolve_edges_ieee(const double* in, const SweepConst* k, const typename M::P* q, double* out) {
+    IeeeDiv dv;
+    evolve_edges_by<M, AXIS>(in, in + M::NU, in + 2 * M::NU, *k, *q, out, out + M::NU, dv);
+}
+template <class M, int AXIS>
+__device__ __noinline__ void force_flux_ieee(const double* in, const SweepConst* k, const typename M::P* q, double* F) {
+    IeeeDiv dv;
+    force_flux_by<M, AXIS>(in, in + M::NU, *k, *q, F, dv);
+}
+template <class M>
+__device__ __noinline__ void cons_ieee(const double* W, const typename M::P* q, double* U) {
+    IeeeDiv dv;
+    cons_by<M>(W, *q, U, dv);
+}
+template <class M>
+__device__ __noinline__ void setcons_ieee(const double* U, const typename M::P* q, double* W) {
+    IeeeDiv dv;
+    setcons_by<M>(U, *q, W, dv);
+}
+
+template <class M, int AXIS>
+__device__ __forceinline__ void evolve_edges(const double* uL, const double* u, const double* uR, const SweepConst& k,
+                                             const typename M::P& q, double* ua_left_side, double* ua_right_side) {
+    if constexpr (shared_div<M>::value) {
+        SharedDiv dv;
+        const bool shared = bias_shared(k.bias);
+        if (shared) evolve_edges_by<M, AXIS>(uL, u, uR, k, q, ua_left_side, ua_right_side, dv);
+        if (!shared || !dv.ok()) {
+            constexpr int NU = M::NU;
+            double in[3 * NU], out[2 * NU];
+            SweepConst kc = k;
+            typename M::P qc = q;
+#pragma unroll
+            for (int i = 0; i < NU; i++) {
+                in[i] = uL[i];
+                in[NU + i] = u[i];
+                in[2 * NU + i] = uR[i];
+            }
+            evolve_edges_ieee<M, AXIS>(in, &kc, &qc, out);
+#pragma unroll
+            for (int i = 0; i < NU; i++) {
+                ua_left_side[i] = out[i];
+                ua_right_side[i] = out[NU + i];
+            }
+        }
+    } else {
+        IeeeDiv dv;
+        evolve_edges_by<M, AXIS>(uL, u, uR, k, q, ua_left_side, ua_right_side, dv);
+    }
+}
+
+template <class M, int AXIS>
+__device__ __forceinline__ void force_flux(const double* ua, const double* ub, const SweepConst& k,
+                                           const typename M::P& q, double* F) {
+    if constexpr (shared_div<M>::value) {
+        SharedDiv dv;
+        force_flux_by<M, AXIS>(ua, ub, k, q, F, dv);
+        if (!dv.ok()) {
+            constexpr int NU = M::NU;
+            double in[2 * NU], out[NU];
+            SweepConst kc = k;
+            typename M::P qc = q;
+#pragma unroll
+            for (int i = 0; i < NU; i++) {
+                in[i] = ua[i];
+                in[NU + i] = ub[i];
+            }
+            force_flux_ieee<M, AXIS>(in, &kc, &qc, out);
+#pragma unroll
+            for (int i = 0; i < NU; i++) F[i] = out[i];
+        }
+    } else {
+        IeeeDiv dv;
+        force_flux_by<M, AXIS>(ua, ub, k, q, F, dv);
+    }
+}
+
+template <class M>
+__device__ __forceinline__ void cons_of(const double* W, const typename M::P& q, double* U) {
+    if constexpr (shared_div<M>::value) {
+        SharedDiv dv;
+        cons_by<M>(W, q, U, dv);
+        if (!dv.ok()) {
+            double w[M::NW], u[M::NU];
+            typename M::P qc = q;
+#pragma unroll
+            for (int i = 0; i < M::NW; i++) w[i] = W[i];
+            cons_ieee<M>(w, &qc, u);
+#pragma unroll
+            for (int i = 0; i < M::NU; i++) U[i] = u[i];
+        }
+    } else {
+        M::cons(W, q, U);
+    }
+}
+
+// W holds the cell's own values of the fields that setConservedVariableVector leaves alone
+template <class M>
+__device__ __forceinline__ void setcons_of(const double* U, const typename M::P& q, double* W) {
+    if constexpr (shared_div<M>::value) {
+        SharedDiv dv;
+        setcons_by<M>(U, q, W, dv);
+        if (!dv.ok()) {
+            double w[M::NW], u[M::NU];
+            typename M::P qc = q;
+#pragma unroll
+            for (int i = 0; i < M::NU; i++) u[i] = U[i];
+#pragma unroll
+            for (int i = 0; i < M::NW; i++) w[i] = W[i];
+            setcons_ieee<M>(u, &qc, w);
+#pragma unroll
+            for (int i = 0; i < M::NW; i++) W[i] = w[i];
+        }
+    } else {
+        M::setcons(U, q, W);
     }
 }
 
@@ -229,7 +413,7 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_kernel(SweepArgs a) {
         int c = ghost_index(s0 - 2 + slot, len, a.periodic);
         double W[NW], U[NU];
         load_w<M>(a, rowbase + c, W);
-        M::cons(W, q, U);
+        cons_of<M>(W, q, U);
 #pragma unroll
         for (int v = 0; v < NU; v++) Us[v][l][slot] = U[v];
     };
@@ -248,7 +432,7 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_kernel(SweepArgs a) {
             u[v] = Us[v][l][p + 1];
             uR[v] = Us[v][l][p + 2];
         }
-        evolve_edges<M, 0>(uL, u, uR, k, q, ub, ua, p >= 1, p <= P - 2);
+        evolve_edges<M, 0>(uL, u, uR, k, q, ub, ua);
 #pragma unroll
         for (int v = 0; v < NU; v++) Es[v][l][p] = ua[v];
     }
@@ -272,7 +456,7 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_kernel(SweepArgs a) {
 #pragma unroll
         for (int v = 0; v < NU; v++) Un[v] = Us[v][l][p + 1] + (k.r * (Fs[v][l][p] - Fs[v][l][p + 1]));
         keep_fields<M>(a, rowbase + cell, q, W);
-        M::setcons(Un, q, W);
+        setcons_of<M>(Un, q, W);
         store_w<M>(a, rowbase + cell, W);
         if (bad_state<M>(W, q)) atomicOr(a.err, ERR_STATE);
         if (a.accumulate_wave) {
@@ -313,7 +497,7 @@ __global__ void __launch_bounds__(TX, MINB) sweep_y_kernel(SweepArgs a) {
         int rr = ghost_index(r, len, a.periodic);
         double W[NW];
         load_w<M>(a, (long)rr * a.pitch + c, W);
-        M::cons(W, q, U);
+        cons_of<M>(W, q, U);
     };
 
     double um1[NU], u0[NU], up1[NU], ua_prev[NU], f_prev[NU], dummy[NU];
@@ -321,11 +505,11 @@ __global__ void __launch_bounds__(TX, MINB) sweep_y_kernel(SweepArgs a) {
     conserve(r0 - 2, up1);   // temporarily holds row r0-2
     conserve(r0 - 1, um1);
     conserve(r0, u0);
-    evolve_edges<M, 1>(up1, um1, u0, k, q, dummy, ua_prev, false, true);   // right edge of row r0-1
+    evolve_edges<M, 1>(up1, um1, u0, k, q, dummy, ua_prev);   // right edge of row r0-1
     for (int r = r0; r <= r1; r++) {
         conserve(r + 1, up1);
         double ub[NU], ua_next[NU];
-        evolve_edges<M, 1>(um1, u0, up1, k, q, ub, ua_next, true, r < r1);
+        evolve_edges<M, 1>(um1, u0, up1, k, q, ub, ua_next);
         double F[NU];
         force_flux<M, 1>(ua_prev, ub, k, q, F);     // flux at r - 1/2
         if (r > r0 && col_ok) {                      // update row r-1 with fluxes at r-3/2 and r-1/2
@@ -333,7 +517,7 @@ __global__ void __launch_bounds__(TX, MINB) sweep_y_kernel(SweepArgs a) {
 #pragma unroll
             for (int v = 0; v < NU; v++) Un[v] = um1[v] + (k.r * (f_prev[v] - F[v]));
             keep_fields<M>(a, (long)(r - 1) * a.pitch + c, q, W);
-            M::setcons(Un, q, W);
+            setcons_of<M>(Un, q, W);
             store_w<M>(a, (long)(r - 1) * a.pitch + c, W);
             if (bad_state<M>(W, q)) atomicOr(a.err, ERR_STATE);
             if (a.accumulate_wave) {

@@ -126,7 +126,7 @@ __global__ void __cluster_dims__(S1D_CL, 1, 1) __launch_bounds__(S1D_NT) solve1d
             double W[NW], U[NU];
 #pragma unroll
             for (int v = 0; v < NW; v++) W[v] = Wsrc[(long)v * seg + (cell - owner * seg)];
-            M::cons(W, q, U);
+            cons_of<M>(W, q, U);
 #pragma unroll
             for (int v = 0; v < NU; v++) Ush[(long)v * (seg + 4) + slot] = U[v];
         }
@@ -145,7 +145,7 @@ __global__ void __cluster_dims__(S1D_CL, 1, 1) __launch_bounds__(S1D_NT) solve1d
                 u[v] = Ush[(long)v * (seg + 4) + cell + 2];
                 uR[v] = Ush[(long)v * (seg + 4) + cell + 3];
             }
-            evolve_edges<M, 0>(uL, u, uR, k, q, ub[kk], ua, cell >= 0, cell <= len - 1);
+            evolve_edges<M, 0>(uL, u, uR, k, q, ub[kk], ua);
 #pragma unroll
             for (int v = 0; v < NU; v++) Esh[(long)v * (seg + 2) + cell + 1] = ua[v];
         }
@@ -177,7 +177,7 @@ __global__ void __cluster_dims__(S1D_CL, 1, 1) __launch_bounds__(S1D_NT) solve1d
                         (k.r * (Fsh[(long)v * (seg + 1) + i] - Fsh[(long)v * (seg + 1) + i + 1]));
 #pragma unroll
             for (int v = 0; v < NW; v++) W[v] = Wb[b][(long)v * seg + i];  // fields setcons leaves alone keep theirs
-            M::setcons(Un, q, W);
+            setcons_of<M>(Un, q, W);
 #pragma unroll
             for (int v = 0; v < NW; v++) Wb[1 - b][(long)v * seg + i] = W[v];
             if (bad_state<M>(W, q)) atomicOr(a.err, ERR_STATE);
