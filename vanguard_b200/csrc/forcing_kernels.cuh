@@ -29,12 +29,11 @@ __device__ __forceinline__ int ghost1_index(int k, int n, int periodic) {
 // evolveStateByFractionalTimeStep (:791-797) on the conserved vectors of the three cells; the result is set into a
 // default-constructed state (primitive out).
 template <class M, int AXIS, class D>
-__device__ __forceinline__ void frac_evolve_u(double frac, const double* uL, const double* uM, const double* uR,
-                                              double dt, double dx, const SweepConst& k, const typename M::P& q,
-                                              double* out, D& dv) {
+__device__ __forceinline__ void frac_evolve_u(double c, const double* uL, double* uM, const double* uR, const SweepConst& k,
+                                              const typename M::P& q, D& dv) {
     constexpr int NU = M::NU;
     double s[NU], xl[NU], xr[NU], fl[NU], fr[NU];
-    slopes_by<NU>(uL, uM, uR, k, s, dv);
+    slopes_by<NU, plain_set<M>::value>(uL, uM, uR, k, s, dv);
 #pragma unroll
     for (int i = 0; i < NU; i++) {
         xl[i] = uM[i] - (0.5 * s[i]);
@@ -42,11 +41,30 @@ __device__ __forceinline__ void frac_evolve_u(double frac, const double* uL, con
     }
     flux_by<M, AXIS>(xl, q, fl, dv);
     flux_by<M, AXIS>(xr, q, fr, dv);
-    double c = frac * (dt / dx);
 #pragma unroll
-    for (int i = 0; i < NU; i++) xl[i] = uM[i] + (c * (fl[i] - fr[i]));
-    M::default_state(out);
-    setcons_by<M>(xl, q, out, dv);
+    for (int i = 0; i < NU; i++) uM[i] = uM[i] + (c * (fl[i] - fr[i]));
+}
+
+// Components that the model's X and Y directions exchange (M::XY_SWAPS): forcing_kernel then runs the Y predictor through
+// the X code, which halves the code of its loop.  The kernel's stalls were a fifth instruction fetches (1.18 of 5.3 cycles per
+// issue at 512^2 HPR).
+template <class M, class = void>
+struct xy_swaps {
+    static constexpr unsigned long long mask = 0;
+};
+template <class M>
+struct xy_swaps<M, decltype((void)M::XY_SWAPS)> {
+    static constexpr unsigned long long mask = M::XY_SWAPS;
+};
+template <class M>
+__device__ __forceinline__ void exchange_xy(double* u, bool yes) {
+#pragma unroll
+    for (int x = 0; x + 1 < M::NU; x++) {
+        if (!(xy_swaps<M>::mask >> x & 1)) continue;
+        const double a = u[x], b = u[x + 1];
+        u[x] = yes ? b : a;
+        u[x + 1] = yes ? a : b;
+    }
 }
 
 // Neighbour round trip of every cell into a.aux (conserved planes): cons -> setConservedVariableVector on a
@@ -119,10 +137,13 @@ __device__ __forceinline__ void forcing_cell(const SweepArgs& a, int subcycles, 
     const double stage_frac[3] = {0.5, 0.5, 1.0};
 #pragma unroll 1
     for (int s = 0; s < 3; s++) {
-        double ut[NU], wm[NW];
-        for (int v = 0; v < NU; v++) ut[v] = uM[v] + (s < 2 ? (0.5 * kk(s, v)) : kk(s, v));
+        double um[NU], wm[NW];
+        for (int v = 0; v < NU; v++) um[v] = uM[v] + (s < 2 ? (0.5 * kk(s, v)) : kk(s, v));
+        // set into a default-constructed state and converted back, here and after each predictor: the two conversions
+        // together share their energy terms
         M::default_state(wm);
-        setcons_by<M>(ut, q, wm, dv);
+        setcons_by<M>(um, q, wm, dv);
+        cons_by<M>(wm, q, um, dv);
         const double f = stage_frac[s];
         // dims == 1: X(f); dims == 2: X(f/2), Y(f), X(f/2)
         const int nsub = dims == 1 ? 1 : 3;
@@ -130,19 +151,28 @@ __device__ __forceinline__ void forcing_cell(const SweepArgs& a, int subcycles, 
         for (int p = 0; p < nsub; p++) {
             const int axis = (dims == 2 && p == 1) ? 1 : 0;
             const double fr = dims == 1 ? f : (p == 1 ? f : 0.5 * f);
-            double uA[NU], uB[NU], um[NU];
+            double uA[NU], uB[NU];
             for (int v = 0; v < NU; v++) {
                 uA[v] = a.aux[v * a.plane + nb[2 * axis]];
                 uB[v] = a.aux[v * a.plane + nb[2 * axis + 1]];
             }
+            const double c = fr * (dt / a.dx);
+            if constexpr (xy_swaps<M>::mask != 0) {
+                exchange_xy<M>(um, axis == 1);
+                exchange_xy<M>(uA, axis == 1);
+                exchange_xy<M>(uB, axis == 1);
+                frac_evolve_u<M, 0>(c, uA, um, uB, k, q, dv);
+                exchange_xy<M>(um, axis == 1);
+            } else if (axis == 0) {
+                frac_evolve_u<M, 0>(c, uA, um, uB, k, q, dv);
+            } else {
+                frac_evolve_u<M, 1>(c, uA, um, uB, k, q, dv);
+            }
+            M::default_state(wm);
+            setcons_by<M>(um, q, wm, dv);
             cons_by<M>(wm, q, um, dv);
-            if (axis == 0)
-                frac_evolve_u<M, 0>(fr, uA, um, uB, dt, a.dx, k, q, wm, dv);
-            else
-                frac_evolve_u<M, 1>(fr, uA, um, uB, dt, a.dx, k, q, wm, dv);
         }
-        cons_by<M>(wm, q, ut, dv);
-        source_by<M>(ut, q, S, dv);
+        source_by<M>(um, q, S, dv);
         if (s < 2)
             for (int v = 0; v < NU; v++) kk(s + 1, v) = dt * S[v];
     }

@@ -15,12 +15,17 @@ namespace vg {
 // ------------------------------------------------------------------------------------------- Euler
 // Stored primitives W = (rho, u, [v], p); conserved U = (rho, rho u, [rho v], E).
 // NVEL = 1 (1D with v == 0) or 2.  Params: params[0] = gamma, params[1] = p_inf.
-template <int NVEL>
+// PLAIN: p_inf == 0 and (in the slopes) no limiter bias, which the launchers check.  The terms that vanish then are left
+// out: x - 0.0 is x, and so is x + 0.0 for the positive pressures that pass the division's range check.
+template <int NVEL, bool PLAIN = false>
 struct EulerF64 {
     static constexpr int NW = NVEL + 2;
     static constexpr int NU = NW;
     static constexpr int IE = NU - 1;  // energy / pressure slot
     static constexpr bool SHARED_DIV = true;
+    static constexpr bool PLAIN_SET = PLAIN;
+    using Plain = EulerF64<NVEL, true>;
+    __device__ __host__ static bool plain(const double* prm) { return prm[1] == 0.0; }
     static constexpr bool HAS_Y = NVEL == 2;
     static constexpr bool HAS_SOURCE = false;
     struct P {
@@ -31,10 +36,12 @@ struct EulerF64 {
     // EulerEquationOfState::computeSpecificInternalEnergy (Euler/eulerequationofstate.cpp:7-13)
     template <class D>
     __device__ static double e_of(double rho, double p, const P& q, D& dv) {
-        return dv.by((q.g - 1) * rho).positive(p + (q.g * q.pinf));
+        return dv.by((q.g - 1) * rho).positive(PLAIN ? p : p + (q.g * q.pinf));
     }
     // EulerEquationOfState::computePressure (Euler/eulerequationofstate.cpp:15-21)
-    __device__ static double p_of(double rho, double e, const P& q) { return ((e * (q.g - 1)) * rho) - (q.g * q.pinf); }
+    __device__ static double p_of(double rho, double e, const P& q) { 
+        return PLAIN ? (e * (q.g - 1)) * rho : ((e * (q.g - 1)) * rho) - (q.g * q.pinf);
+    }
 
     __device__ static double vsq(double u, double v) {
         if constexpr (NVEL == 2) return (u * u) + (v * v);
@@ -122,7 +129,7 @@ struct EulerF64 {
 // FULL: W = (rho, u, v, w, p, Bx, By, Bz, psi), U = (rho, mx, my, mz, E, Bx, By, Bz, psi).
 // reduced: W = (rho, u, v, p, Bx, By, psi),    U = (rho, mx, my, E, Bx, By, psi)   (w == Bz == 0).
 // Params: params[0] = gamma, params[1] = p_inf; c_h comes from the control block each step.
-template <bool FULL>
+template <bool FULL, bool PLAIN = false>
 struct MHDF64 {
     static constexpr int NW = FULL ? 9 : 7;
     static constexpr int NU = NW;
@@ -131,6 +138,11 @@ struct MHDF64 {
     static constexpr int IBY = IP + 2;
     static constexpr int IPSI = NW - 1;
     static constexpr bool SHARED_DIV = true;
+    static constexpr bool PLAIN_SET = PLAIN;
+    using Plain = MHDF64<FULL, true>;
+    __device__ __host__ static bool plain(const double* prm) { return prm[1] == 0.0; }
+    // see HPRModel::XY_SWAPS: mx my, Bx By
+    static constexpr unsigned long long XY_SWAPS = 1ull << 1 | 1ull << (FULL ? 5 : 4);
     static constexpr bool HAS_Y = true;
     static constexpr bool HAS_SOURCE = true;
     struct P {
@@ -154,9 +166,11 @@ struct MHDF64 {
 
     template <class D>
     __device__ static double e_of(double rho, double p, const P& q, D& dv) {
-        return dv.by((q.g - 1) * rho).positive(p + (q.g * q.pinf));
+        return dv.by((q.g - 1) * rho).positive(PLAIN ? p : p + (q.g * q.pinf));
     }
-    __device__ static double p_of(double rho, double e, const P& q) { return ((e * (q.g - 1)) * rho) - (q.g * q.pinf); }
+    __device__ static double p_of(double rho, double e, const P& q) { 
+        return PLAIN ? (e * (q.g - 1)) * rho : ((e * (q.g - 1)) * rho) - (q.g * q.pinf);
+    }
 
     __device__ static double sq3(double a, double b, double c) {
         if constexpr (FULL) return ((a * a) + (b * b)) + (c * c);
@@ -283,10 +297,14 @@ struct MHDF64 {
 // W = (alpha1, u, v, rho1, rho2, p), U = (rho, rho alpha1, rho u, rho v, alpha1 rho1, alpha2 rho2, rho E).
 // Params: {gamma1, p_inf1, gamma2, p_inf2}.  Every volume fraction the model derives or uses is clamped to
 // [0.001, 0.999] (:47-58, :99-108, :131-147).
-struct EulerReducedF64 {
+template <bool PLAIN = false>
+struct EulerReducedModel {
     static constexpr int NW = 6;
     static constexpr int NU = 7;
     static constexpr bool SHARED_DIV = true;
+    static constexpr bool PLAIN_SET = PLAIN;
+    using Plain = EulerReducedModel<true>;
+    __device__ __host__ static bool plain(const double* prm) { return prm[1] == 0.0 && prm[3] == 0.0; }
     static constexpr bool HAS_Y = true;
     static constexpr bool HAS_SOURCE = false;
     struct P {
@@ -303,13 +321,15 @@ struct EulerReducedF64 {
     // (Euler/eulerequationofstate.cpp:7-29) of material (g, pinf)
     template <class D>
     __device__ static double e_of(double rho, double p, double g, double pinf, D& dv) {
-        return dv.by((g - 1) * rho).positive(p + (g * pinf));
+        return dv.by((g - 1) * rho).positive(PLAIN ? p : p + (g * pinf));
     }
     __device__ static double e_of(double rho, double p, double g, double pinf) {
         IeeeDiv dv;
         return e_of(rho, p, g, pinf, dv);
     }
-    __device__ static double p_of(double rho, double e, double g, double pinf) { return ((e * (g - 1)) * rho) - (g * pinf); }
+    __device__ static double p_of(double rho, double e, double g, double pinf) { 
+        return PLAIN ? (e * (g - 1)) * rho : ((e * (g - 1)) * rho) - (g * pinf);
+    }
     __device__ static double c_of(double rho, double p, double g, double pinf) { return sqrt((g * (p + pinf)) / rho); }
 
     // EulerReducedStateVector::computeConservedVariableVector (:96-129)
@@ -398,6 +418,7 @@ struct EulerReducedF64 {
     __device__ static double density(const double* W) { return W[3] < W[4] ? W[3] : W[4]; }
     __device__ static double pressure(const double* W) { return W[5]; }
 };
+using EulerReducedF64 = EulerReducedModel<>;
 
 // ------------------------------------------------------------------------- Euler multiphysics two-material
 // EulerMultiphysicsStateVector (Euler/Multiphysics/eulermultiphysicsstatevector.cpp) with w == 0 (host-checked):
@@ -499,10 +520,15 @@ struct EulerMultiphysicsF64 {
 // materials, is this step's maximum wave speed as MHDSecondOrderSolver::solve{,2D} sets it (Solvers/
 // mhdsecondordersolver.cpp:454-460), with the parabolic damping c_p = sqrt(c_h * 0.18) (MHD/mhdmaterialparameters.cpp:
 // 31-34).  The GLM coefficients enter as the volume-fraction mixtures of c_h^2 and c_p^2, as the reference forms them.
-struct MHDReducedF64 {
+template <bool PLAIN = false>
+struct MHDReducedModel {
     static constexpr int NW = 11;
     static constexpr int NU = 12;
     static constexpr bool SHARED_DIV = true;
+    static constexpr bool PLAIN_SET = PLAIN;
+    using Plain = MHDReducedModel<true>;
+    __device__ __host__ static bool plain(const double* prm) { return prm[1] == 0.0 && prm[3] == 0.0; }
+    static constexpr unsigned long long XY_SWAPS = 1ull << 2 | 1ull << 8;  // see HPRModel::XY_SWAPS: rho u rho v, Bx By
     static constexpr bool HAS_Y = true;
     static constexpr bool HAS_SOURCE = true;
     // GLM forcing at 8 resident blocks (128 registers): 7.6 % faster per 2048^2 step than at 6, same bits
@@ -516,7 +542,7 @@ struct MHDReducedF64 {
     }
     // clamp_alpha and the stiffened-gas e(rho, p) / p(rho, e) of MHDEquationOfState (MHD/mhdequationofstate.cpp:7-21),
     // which are EulerEquationOfState's
-    using R2 = EulerReducedF64;
+    using R2 = EulerReducedModel<PLAIN>;
 
     __device__ static double b2_of(double bx, double by, double bz) { return ((bx * bx) + (by * by)) + (bz * bz); }
 
@@ -666,6 +692,7 @@ struct MHDReducedF64 {
     __device__ static double density(const double* W) { return W[4] < W[5] ? W[4] : W[5]; }
     __device__ static double pressure(const double* W) { return W[6]; }
 };
+using MHDReducedF64 = MHDReducedModel<>;
 
 // ------------------------------------------------------------------------ MHD intermediate two-material
 // MHDIntermediateStateVector (MHD/Multiphysics/mhdintermediatestatevector.cpp), every plane carried:

@@ -19,6 +19,8 @@
 //           sigma0, n}
 #pragma once
 
+#include <type_traits>
+
 #include "exact_div.cuh"
 #include "vg_common.cuh"
 
@@ -27,8 +29,18 @@ namespace vg {
 // SOLID = false: the StiffenedGas gas with elastic strain relaxation only (the thermal-gas configurations);
 // SOLID = true: every equation-of-state branch (params[12]) and the plastic relaxation (params[17]).  The gas
 // instantiation compiles the StiffenedGas formulas alone, so it carries no branch or register cost for solids.
-template <bool SOLID>
+// PLAIN: p_inf == 0 and (in the slopes) no limiter bias, which the launchers check; the terms that vanish then are left out
+// (x + 0.0 and x - 0.0 are x for the positive x they are applied to; any other fails the division's range check).
+template <bool SOLID, bool PLAIN = false>
 struct HPRModel {
+    static constexpr bool PLAIN_SET = PLAIN;
+    using Plain = HPRModel<SOLID, !SOLID>;
+    __device__ __host__ static bool plain(const double* prm) { return !SOLID && prm[1] == 0.0; }
+    // components that trade places between the X and the Y direction: the flux along Y of a state is the flux along X of the
+    // state with these exchanged, exchanged back, bit for bit (every sum that is reordered is one of two terms, or the first
+    // two of three)
+    // bit i: component i with its successor: A00 A01, A10 A11, A20 A21, u v, Jx Jy
+    static constexpr unsigned long long XY_SWAPS = 1ull << 2 | 1ull << 5 | 1ull << 8 | 1ull << 11 | 1ull << 14;
     static constexpr int NW = 17;
     static constexpr int NU = 17;
     static constexpr bool SHARED_DIV = !SOLID;  // the solid equations of state divide as the compiler does
@@ -61,12 +73,17 @@ struct HPRModel {
             for (int j = 0; j < 3; j++) r.m[i][j] = a9[3 * i + j];
         return r;
     }
+    // a sum of three products from 0.0, as MatrixAlgebra and VectorAlgebra form it: 0.0 + x y in one operation, which
+    // rounds x y as the product alone does
+    __device__ static double dot3(double a0, double b0, double a1, double b1, double a2, double b2) {
+        return (__fma_rn(a0, b0, 0.0) + (a1 * b1)) + (a2 * b2);
+    }
     __device__ static M3 mul(const M3& a, const M3& b) {
         M3 r;
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) r.m[i][j] = ((0.0 + (a.m[i][0] * b.m[0][j])) + (a.m[i][1] * b.m[1][j])) + (a.m[i][2] * b.m[2][j]);
+            for (int j = 0; j < 3; j++) r.m[i][j] = dot3(a.m[i][0], b.m[0][j], a.m[i][1], b.m[1][j], a.m[i][2], b.m[2][j]);
         return r;
     }
     __device__ static M3 tmul(const M3& a, const M3& b) {  // a^T b
@@ -74,7 +91,7 @@ struct HPRModel {
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) r.m[i][j] = ((0.0 + (a.m[0][i] * b.m[0][j])) + (a.m[1][i] * b.m[1][j])) + (a.m[2][i] * b.m[2][j]);
+            for (int j = 0; j < 3; j++) r.m[i][j] = dot3(a.m[0][i], b.m[0][j], a.m[1][i], b.m[1][j], a.m[2][i], b.m[2][j]);
         return r;
     }
     // TensorAlgebra::computeDeviator (Mathematics/tensoralgebra.cpp:27-30)
@@ -85,7 +102,12 @@ struct HPRModel {
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) r.m[i][j] = g.m[i][j] + (-1.0 * (c * (i == j ? 1.0 : 0.0)));
+            for (int j = 0; j < 3; j++) {
+                // off the diagonal the reference adds -(c * 0.0), which is -0.0 for the finite, non-negative mean of a
+                // Gram matrix's diagonal and changes nothing
+                if (std::is_same<D, SharedDiv>::value && i != j) r.m[i][j] = g.m[i][j];
+                else r.m[i][j] = g.m[i][j] + (-1.0 * (c * (i == j ? 1.0 : 0.0)));
+            }
         return r;
     }
     __device__ static M3 dev(const M3& g) {
@@ -107,6 +129,7 @@ struct HPRModel {
     }
     __device__ static double gr_coef(double rho, const P& q) { return pow((rho / q.rho0), q.aeos); }
     __device__ static double mg_pref(double rho, const P& q) {  // computeReferencePressure (:30-66)
+        if constexpr (PLAIN) return -0.0;
         if constexpr (!SOLID) return -q.pinf;
         if (q.eos == 1) {
             double c0sq = q.c0 * q.c0;
@@ -126,6 +149,7 @@ struct HPRModel {
     }
     template <class By>
     __device__ static double mg_eref(double rho, const P& q, const By& by_rho) {
+        if constexpr (PLAIN) return 0.0;
         if constexpr (!SOLID) return by_rho(q.pinf);
         if (q.eos == 1) return rho > q.rho0 ? (0.5 * q.pref_mat) * ((1.0 / q.rho0) - (1.0 / rho)) : 0.0;
         if (q.eos == 2) {
@@ -166,14 +190,17 @@ struct HPRModel {
     // computeInternalEnergy / computePressure / computeTemperature (:194-221)
     template <class D>
     __device__ static double mg_energy(double rho, double p, const P& q, D& dv) {
+        if constexpr (PLAIN) return dv.by(rho * mg_G(rho, q)).positive(p);
         return mg_eref(rho, q, dv.by(rho)) + dv.by(rho * mg_G(rho, q)).positive(p - mg_pref(rho, q));
     }
     template <class By>
     __device__ static double mg_pressure(double rho, double e, const P& q, const By& by_rho) {
+        if constexpr (PLAIN) return (e * rho) * mg_G(rho, q);
         return (((e - mg_eref(rho, q, by_rho)) * rho) * mg_G(rho, q)) + mg_pref(rho, q);
     }
     template <class D>
     __device__ static double mg_temperature(double rho, double p, const P& q, D& dv) {
+        if constexpr (PLAIN) return q.Tref + dv.by((rho * mg_G(rho, q)) * q.cv).positive(p);
         return q.Tref + dv.by((rho * mg_G(rho, q)) * q.cv).positive(p - mg_pref(rho, q));
     }
     __device__ static double mg_temperature(double rho, double p, const P& q) {
@@ -198,7 +225,7 @@ struct HPRModel {
         M3 D = dev(tmul(A, A), dv);
         double sum = 0.0;
 #pragma unroll
-        for (int i = 0; i < 3; i++) sum += ((0.0 + (D.m[i][0] * D.m[i][0])) + (D.m[i][1] * D.m[i][1])) + (D.m[i][2] * D.m[i][2]);
+        for (int i = 0; i < 3; i++) sum += dot3(D.m[i][0], D.m[i][0], D.m[i][1], D.m[i][1], D.m[i][2], D.m[i][2]);
         return (0.25 * (q.cs * q.cs)) * sum;
     }
     __device__ static double meso_thermal(double jx, double jy, double jz, const P& q) {
@@ -310,11 +337,11 @@ struct HPRModel {
             F[12] = (rho * (v * v)) + p;
             F[13] = rho * (v * w);
         }
-        F[1] -= ((0.0 + (sig[0] * u)) + (sig[1] * v)) + (sig[2] * w);
+        F[1] -= dot3(sig[0], u, sig[1], v, sig[2], w);
 #pragma unroll
         for (int i = 0; i < 3; i++) F[11 + i] -= sig[i];
 #pragma unroll
-        for (int i = 0; i < 3; i++) F[2 + (i * 3) + AXIS] = ((0.0 + (A.m[i][0] * u)) + (A.m[i][1] * v)) + (A.m[i][2] * w);
+        for (int i = 0; i < 3; i++) F[2 + (i * 3) + AXIS] = dot3(A.m[i][0], u, A.m[i][1], v, A.m[i][2], w);
         if (q.thermal) {
             double T = mg_temperature(rho, p, q, dv);
             double a2 = q.alpha * q.alpha;

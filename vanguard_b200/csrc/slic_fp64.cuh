@@ -24,7 +24,7 @@ constexpr int MW_NT = 256;
 struct Fp64Kernels {
     template <class M, int P, int LPB, int MINB>
     static void x(dim3 grid, int nt, cudaStream_t st, const SweepArgs& a) {
-        sweep_x_kernel<M, P, LPB, MINB><<<grid, nt, 0, st>>>(a);
+        plain_form<M>::pick(a, [&](auto m) { sweep_x_kernel<decltype(m), P, LPB, MINB><<<grid, nt, 0, st>>>(a); });
     }
     template <class M, int TX, int TY, int MINB>
     static int y_resident() {
@@ -34,7 +34,7 @@ struct Fp64Kernels {
     }
     template <class M, int TX, int TY, int MINB>
     static void y(dim3 grid, int nt, cudaStream_t st, const SweepArgs& a) {
-        sweep_y_kernel<M, TX, TY, MINB><<<grid, nt, 0, st>>>(a);
+        plain_form<M>::pick(a, [&](auto m) { sweep_y_kernel<decltype(m), TX, TY, MINB><<<grid, nt, 0, st>>>(a); });
     }
 };
 
@@ -65,7 +65,9 @@ cudaError_t forcing_impl(const SweepArgs& a, int subcycles, cudaStream_t st) {
     if (!a.aux) return cudaErrorInvalidValue;
     long n = (long)a.nx * a.ny;
     roundtrip_kernel<M><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a);
-    forcing_kernel<M><<<(unsigned)((n + FT - 1) / FT), FT, sizeof(double) * 3 * M::NU * FT, st>>>(a, subcycles);
+    plain_form<M>::pick(a, [&](auto m) {
+        forcing_kernel<decltype(m)><<<(unsigned)((n + FT - 1) / FT), FT, sizeof(double) * 3 * M::NU * FT, st>>>(a, subcycles);
+    });
     return cudaGetLastError();
 }
 

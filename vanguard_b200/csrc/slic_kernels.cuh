@@ -31,6 +31,31 @@ template <class M>
 struct shared_div<M, decltype((void)M::SHARED_DIV)> {
     static constexpr bool value = M::SHARED_DIV;
 };
+// Models compiled once more for p_inf == 0 and no limiter bias (M::Plain) say in which of the two forms they are.
+template <class M, class = void>
+struct plain_set {
+    static constexpr bool value = false;
+};
+template <class M>
+struct plain_set<M, decltype((void)M::PLAIN_SET)> {
+    static constexpr bool value = M::PLAIN_SET;
+};
+// f(M::Plain{}) where the model has that form and the launch's parameters allow it, f(M{}) otherwise
+template <class M, class = void>
+struct plain_form {
+    template <class F>
+    static auto pick(const SweepArgs&, F f) {
+        return f(M{});
+    }
+};
+template <class M>
+struct plain_form<M, std::enable_if_t<!plain_set<M>::value && plain_set<typename M::Plain>::value>> {
+    template <class F>
+    static auto pick(const SweepArgs& a, F f) {
+        return a.bias == 0.0 && M::plain(a.params) ? f(typename M::Plain{}) : f(M{});
+    }
+};
+
 template <class M, class D>
 __device__ __forceinline__ void cons_by(const double* W, const typename M::P& q, double* U, D& dv) {
     if constexpr (shared_div<M>::value) M::cons(W, q, U, dv);
@@ -67,49 +92,61 @@ __device__ __forceinline__ double limiter_f64(double r, double w, int id) {
 // is formed, and the ones that the reference's branch does not reach are not used.  r is compared with 0, 1/2 and 1 by
 // its upper word (the constants' lower words are zero).  For r >= 1 the second divisor is at least 2 to within a
 // rounding, so xi_R stays below 2 and the reference's outer minimum with 2 cannot bite.
-template <int ID>
+// UNBIASED (w == 0): the divisor is 1 + r exactly as the reference rounds it, both quotients of van Leer's limiter share its
+// reciprocal, and xi_R <= 1 <= r for r >= 1 decides the other minima.
+template <int ID, bool UNBIASED>
 __device__ __forceinline__ double limiter_shared(double r, double w) {
     const int hi = __double2hiint(r);
     const bool low = hi < 0x3ff00000;
-    const double xi = SharedDiv::known(2.0, (1.0 - w) + ((1.0 + w) * r));
     double phi;
-    if constexpr (ID == 0)
-        phi = low ? (hi < 0x3fe00000 ? 2.0 * r : 1.0) : std_min(r, xi);
-    else if constexpr (ID == 1)
-        phi = std_min(SharedDiv::known(2.0 * r, 1.0 + r), xi);
-    else
-        phi = low ? r : std_min(1.0, xi);
+    if constexpr (UNBIASED) {
+        const double b = 1.0 + r, y = SharedDiv::reciprocal(b);
+        const double xi = SharedDiv::quotient(2.0, b, y);
+        if constexpr (ID == 0) phi = low ? (hi < 0x3fe00000 ? 2.0 * r : 1.0) : xi;
+        else if constexpr (ID == 1) phi = std_min(SharedDiv::quotient(2.0 * r, b, y), xi);
+        else phi = low ? r : xi;
+    } else {
+        const double xi = SharedDiv::known(2.0, (1.0 - w) + ((1.0 + w) * r));
+        if constexpr (ID == 0) phi = low ? (hi < 0x3fe00000 ? 2.0 * r : 1.0) : std_min(r, xi);
+        else if constexpr (ID == 1) phi = std_min(SharedDiv::known(2.0 * r, 1.0 + r), xi);
+        else phi = low ? r : std_min(1.0, xi);
+    }
     return hi < 0 ? 0.0 : phi;
+}
+
+// |d| < floor5 by the bit patterns (which order as the magnitudes do; a NaN is above): the FP64 pipe is what the sweeps run
+// out of
+__device__ __forceinline__ double floored(double d, double floor5) {
+    const unsigned long long m = (unsigned long long)__double_as_longlong(d) & 0x7fffffffffffffffULL;
+    return m < (unsigned long long)__double_as_longlong(floor5) ? floor5 : d;
 }
 
 // SlopeLimiters::computeSlopeVector (Solvers/slopelimiters.cpp:217-246) of n components.  The limiter is chosen outside
 // the loop, so that the components' chains of divisions overlap.
-template <int ID, int N, class D>
+template <int ID, int N, bool UNBIASED, class D>
 __device__ __forceinline__ void slopes_of(const double* uL, const double* u, const double* uR, const SweepConst& k,
                                           double* s, D& dv) {
 #pragma unroll
     for (int i = 0; i < N; i++) {
         const double dm = u[i] - uL[i], dp = uR[i] - u[i];
-        double num = dm, den = dp;
-        if (fabs(num) < k.floor5) num = k.floor5;
-        if (fabs(den) < k.floor5) den = k.floor5;
+        const double num = floored(dm, k.floor5), den = floored(dp, k.floor5);
         double phi;
         if constexpr (std::is_same<D, SharedDiv>::value) {
             dv.note_below(dm);
             dv.note_below(dp);
-            phi = limiter_shared<ID>(SharedDiv::known(num, den), k.bias);
+            phi = limiter_shared<ID, UNBIASED>(SharedDiv::known(num, den), k.bias);
         } else {
             phi = limiter_f64(num / den, k.bias, ID);
         }
         s[i] = ((k.cm * dm) + (k.cp * dp)) * phi;
     }
 }
-template <int N, class D>
+template <int N, bool UNBIASED, class D>
 __device__ __forceinline__ void slopes_by(const double* uL, const double* u, const double* uR, const SweepConst& k,
                                           double* s, D& dv) {
-    if (k.limiter == 0) slopes_of<0, N>(uL, u, uR, k, s, dv);
-    else if (k.limiter == 1) slopes_of<1, N>(uL, u, uR, k, s, dv);
-    else slopes_of<2, N>(uL, u, uR, k, s, dv);
+    if (k.limiter == 0) slopes_of<0, N, UNBIASED>(uL, u, uR, k, s, dv);
+    else if (k.limiter == 1) slopes_of<1, N, UNBIASED>(uL, u, uR, k, s, dv);
+    else slopes_of<2, N, UNBIASED>(uL, u, uR, k, s, dv);
 }
 // whether the branch-free limiter covers this bias
 __device__ __forceinline__ bool bias_shared(double w) { return fabs(w) <= 1.0; }
@@ -122,7 +159,7 @@ __device__ __forceinline__ void evolve_edges_by(const double* uL, const double* 
                                                 const typename M::P& q, double* ua_left_side, double* ua_right_side, D& dv) {
     constexpr int NU = M::NU;
     double s[NU], xl[NU], xr[NU], fl[NU], fr[NU];
-    slopes_by<NU>(uL, u, uR, k, s, dv);
+    slopes_by<NU, plain_set<M>::value>(uL, u, uR, k, s, dv);
 #pragma unroll
     for (int i = 0; i < NU; i++) {
         xl[i] = u[i] - (0.5 * s[i]);
@@ -500,14 +537,17 @@ __global__ void __launch_bounds__(TX, MINB) sweep_y_kernel(SweepArgs a) {
         cons_of<M>(W, q, U);
     };
 
-    double um1[NU], u0[NU], up1[NU], ua_prev[NU], f_prev[NU], dummy[NU];
+    double um1[NU], u0[NU], up1[NU], ua_prev[NU], f_prev[NU], dummy[NU], next[NW];
     double wave = 0.0;
+    auto fetch = [&](int r) { load_w<M>(a, (long)ghost_index(r, len, a.periodic) * a.pitch + c, next); };
     conserve(r0 - 2, up1);   // temporarily holds row r0-2
     conserve(r0 - 1, um1);
     conserve(r0, u0);
+    fetch(r0 + 1);  // one row ahead of its use
     evolve_edges<M, 1>(up1, um1, u0, k, q, dummy, ua_prev);   // right edge of row r0-1
     for (int r = r0; r <= r1; r++) {
-        conserve(r + 1, up1);
+        cons_of<M>(next, q, up1);
+        fetch(r + 2);
         double ub[NU], ua_next[NU];
         evolve_edges<M, 1>(um1, u0, up1, k, q, ub, ua_next);
         double F[NU];
