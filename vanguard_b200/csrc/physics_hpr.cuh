@@ -73,10 +73,11 @@ struct HPRModel {
             for (int j = 0; j < 3; j++) r.m[i][j] = a9[3 * i + j];
         return r;
     }
-    // a sum of three products from 0.0, as MatrixAlgebra and VectorAlgebra form it: 0.0 + x y in one operation, which
-    // rounds x y as the product alone does
+    // a sum of three products from 0.0, as MatrixAlgebra and VectorAlgebra form it; the plain form takes 0.0 + x y in one
+    // operation, which rounds x y as the product alone does
     __device__ static double dot3(double a0, double b0, double a1, double b1, double a2, double b2) {
-        return (__fma_rn(a0, b0, 0.0) + (a1 * b1)) + (a2 * b2);
+        if constexpr (PLAIN) return (__fma_rn(a0, b0, 0.0) + (a1 * b1)) + (a2 * b2);
+        else return ((0.0 + (a0 * b0)) + (a1 * b1)) + (a2 * b2);
     }
     __device__ static M3 mul(const M3& a, const M3& b) {
         M3 r;

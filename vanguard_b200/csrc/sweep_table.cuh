@@ -5,6 +5,7 @@
 // the autotuner (vg_autotune in vg_api.cu) times them on the caller's grid and keeps the fastest.
 #pragma once
 
+#include <algorithm>
 #include <atomic>
 
 #include <cuda_runtime.h>
@@ -27,19 +28,25 @@ cudaError_t launch_x(const SweepArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Rows marched per Y-sweep block when segments are sized for whole waves.  A grid of a few waves leaves its last wave
-// mostly empty (2048 blocks on 888 resident slots run as three waves), so the segment length is chosen from TY / 2 to
-// 4 TY to minimise waves x (rows + 3), the 3 being the rows a block spends starting its march.  Whether that beats
-// the shape's own TY depends on the model (measured: MHD Y sweeps 7-14 % faster, Euler's up to 5 % slower), so the
-// autotuner times every shape both ways.  The results do not depend on the segmentation.
-inline int y_segment_rows(int ny, int xblocks, long slots, int ty0) {
-    if (slots <= 0 || ny <= 0) return ty0;
+// Rows marched per Y-sweep block when segments are sized for the device: the segment length from 2 to 4 TY that minimises
+// the time of the grid in units of one warp's row.  A scheduler with w resident warps takes max(latency, w) such units for a
+// row of all of them (latency: one warp's row alone against its share of a busy pipe), a block starts its march with about
+// 2.3 rows, every full wave of resident blocks runs at the full w, and the last one at what its blocks give each SM.  Measured
+// on the exact form, whose one warp per scheduler takes 1.4 of its pipe time (130 x 97 Euler: 35 us a sweep with the shape's
+// 64 rows, 9 us with 2; 2048^2 MHD: 0.296 ms with 64 rows, 0.253 ms with 32); the mixed form has shorter rows to hide the
+// same latency with.  The results do not depend on the segmentation.  The autotuner times every shape both ways.
+inline int y_segment_rows(int ny, int xblocks, int tx, long slots, int sms, double latency, int ty0) {
+    if (slots <= 0 || sms <= 0 || ny <= 0) return ty0;
+    const double warps = tx / 32.0 / 4.0;  // of one block on each scheduler
+    const double full = std::max(latency, (double)(slots / sms) * warps);
     int best = ty0;
     double best_cost = 1e300;
-    for (int ty = (ty0 + 1) / 2; ty <= 4 * ty0; ty++) {
+    for (int ty = 2; ty <= 4 * ty0; ty++) {
         const long blocks = (long)xblocks * ((ny + ty - 1) / ty);
-        const long waves = (blocks + slots - 1) / slots;
-        const double cost = (double)waves * (double)(ty + 3);
+        const long waves = blocks / slots, rest = blocks % slots;
+        double cost = (double)waves * full;
+        if (rest) cost += std::max(latency, (double)((rest + sms - 1) / sms) * warps);
+        cost *= ty + 2.3;
         if (cost < best_cost) {
             best_cost = cost;
             best = ty;
@@ -56,19 +63,22 @@ cudaError_t launch_y(const SweepArgs& a0, cudaStream_t st) {
         return cudaErrorInvalidValue;
     } else {
         static std::atomic<long> cached{0};  // resident blocks of this shape on the device (every thread stores the same)
-        long slots = cached.load(std::memory_order_relaxed);
+        static std::atomic<int> cached_sms{0};
+        long slots = cached.load(std::memory_order_acquire);
         if (slots == 0) {
-            int dev = 0, sms = 0;
+            int dev = 0, n = 0;
             cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            slots = (long)K::template y_resident<M, TX, TY, MINB>() * sms;
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+            slots = (long)K::template y_resident<M, TX, TY, MINB>() * n;
             if (slots <= 0) slots = -1;
-            cached.store(slots, std::memory_order_relaxed);
+            cached_sms.store(n, std::memory_order_relaxed);
+            cached.store(slots, std::memory_order_release);
         }
+        const int sms = cached_sms.load(std::memory_order_relaxed);
         if (a0.nx <= 0) return cudaSuccess;  // a call that only looks the occupancy up (before a graph capture)
         SweepArgs a = a0;
         const int xblocks = (a.nx + TX - 1) / TX;
-        a.ty_rows = a.y_waves ? y_segment_rows(a.ny, xblocks, slots, TY) : TY;
+        a.ty_rows = a.y_waves ? y_segment_rows(a.ny, xblocks, TX, slots, sms, K::ROW_LATENCY, TY) : TY;
         dim3 grid(xblocks, (a.ny + a.ty_rows - 1) / a.ty_rows);
         K::template y<M, TX, TY, MINB>(grid, TX, st, a);
         return cudaGetLastError();
@@ -94,6 +104,18 @@ struct pair_sweeps<M, decltype((void)M::PAIR_X)> {
     static constexpr bool value = M::PAIR_X;
 };
 
+// The exact-form models with shared reciprocals (exact_div.cuh) have long independent chains that the compiler would overlap
+// with every register it can get; their own tables cap the registers where more resident warps pay more (kinds 5 and 6,
+// index 0 the default).
+template <class M, class = void>
+struct shared_sweeps {
+    static constexpr bool value = false;
+};
+template <class M>
+struct shared_sweeps<M, decltype((void)M::SHARED_DIV)> {
+    static constexpr bool value = M::SHARED_DIV;
+};
+
 // Models with more than 9 conserved components (HPR, 17) use shorter X segments so that the three FP64
 // shared-memory tiles stay inside the 48 KB static limit (kind 1); models with more than 21 (the HPR multiphysics
 // model, 33) shorter still (kind 4).  The PAIR_X models (two rows per thread in the X sweep) add the TMA-staged X
@@ -101,7 +123,8 @@ struct pair_sweeps<M, decltype((void)M::PAIR_X)> {
 // (kind 3).
 template <class M>
 constexpr int tile_kind() {
-    return (M::NU > 21) ? 4 : (M::NU > 9) ? 1 : pair_sweeps<M>::value ? (M::NW <= 4 ? 2 : 3) : 0;
+    return (M::NU > 21) ? 4 : (M::NU > 9) ? (shared_sweeps<M>::value ? 5 : 1) : pair_sweeps<M>::value ? (M::NW <= 4 ? 2 : 3)
+           : shared_sweeps<M>::value ? 6 : 0;
 }
 
 template <class K, class M, int KIND = tile_kind<M>()>
@@ -167,6 +190,37 @@ struct SweepTable<K, M, 3> {
     };
 };
 
+// X, measured in ms a sweep (4096^2 Euler | 2048^2 MHD7 | 2048^2 two-material Euler | 2048^2 MHD9): 7 blocks of 128 (72
+// registers) 0.648 | 0.266 | 0.335 | -, 5 (96) 0.689 | 0.264 | 0.332 | 0.403, 4 (128) 0.730 | 0.271 | 0.337 | 0.339, no cap 0.73 |
+// 0.38 | 0.45 | 0.36.  Y: 8 blocks of 64 (128 registers) 0.606 for Euler against 0.616 without a cap; the longer states lose
+// more to spills than the warps give (MHD7 0.291 against 0.253, two-material Euler 0.358 against 0.344).
+template <class K, class M>
+struct SweepTable<K, M, 6> {
+    static constexpr int XB = M::NU <= 7 ? 7 : 4, YB = M::NU <= 4 ? 8 : 1;
+    static constexpr SweepFn x[kNumXCfg] = {
+        launch_x<K, M, 128, 1, XB>, launch_x<K, M, 64, 1, 9>, launch_x<K, M, 96, 1, 8>,
+        launch_x<K, M, 128, 1, 5>, launch_x<K, M, 128, 1, 8>,
+    };
+    static constexpr SweepFn y[kNumYCfg] = {
+        launch_y<K, M, 64, 64, YB>, launch_y<K, M, 64, 32, 5>, launch_y<K, M, 64, 64, 12>,
+        launch_y<K, M, 64, 64, 10>, launch_y<K, M, 128, 32, 1>, launch_y<K, M, 32, 64, YB>,
+    };
+};
+
+// X (1001x777 two-material MHD | 1024^2 HPR): 4 blocks of 96 (168 registers) 0.118 | 0.271, 5 of 64 (168) 0.119 | 0.291, no cap
+// 0.135 | 0.288.
+template <class K, class M>
+struct SweepTable<K, M, 5> {
+    static constexpr SweepFn x[kNumXCfg] = {
+        launch_x<K, M, 96, 1, 4>, launch_x<K, M, 64, 1, 5>, launch_x<K, M, 64, 1, 1>,
+        launch_x<K, M, 32, 2, 5>, launch_x<K, M, 32, 1, 1>,
+    };
+    static constexpr SweepFn y[kNumYCfg] = {
+        launch_y<K, M, 64, 64, 1>, launch_y<K, M, 64, 32, 1>, launch_y<K, M, 32, 32, 1>,
+        launch_y<K, M, 32, 64, 1>, launch_y<K, M, 128, 32, 1>, launch_y<K, M, 64, 16, 5>,
+    };
+};
+
 // Names of the shapes of SweepTable<K, M, kind>.
 inline const char* x_cfg_name(int i, int kind = 0) {
     static const char* n[kNumXCfg] = {"P128xL1", "P64xL2", "P192xL1", "P128xL1/min6", "P128xL1/min8"};
@@ -174,15 +228,21 @@ inline const char* x_cfg_name(int i, int kind = 0) {
     static const char* np[kNumXCfg] = {"P128x2", "TMA P128x2/min7", "TMA P128x2/min8", "P128x2/min6", "P128x2/min8"};
     static const char* nq[kNumXCfg] = {"P128x2", "P64xL2x2", "P128x2/min4", "P128x2/min6", "P128x2/min8"};
     static const char* nw[kNumXCfg] = {"P32xL1", "P40xL1", "P48xL1", "P56xL1", "P32xL1/min2"};
+    static const char* ns[kNumXCfg] = {"P128xL1", "P64xL1/min9", "P96xL1/min8", "P128xL1/min5", "P128xL1/min8"};
+    static const char* nt[kNumXCfg] = {"P96xL1/min4", "P64xL1/min5", "P64xL1", "P32xL2/min5", "P32xL1"};
     return (i >= 0 && i < kNumXCfg)
-               ? (kind == 1 ? nb[i] : kind == 2 ? np[i] : kind == 3 ? nq[i] : kind == 4 ? nw[i] : n[i])
+               ? (kind == 5 ? nt[i] : kind == 6 ? ns[i] : kind == 1 ? nb[i] : kind == 2 ? np[i] : kind == 3 ? nq[i] : kind == 4 ? nw[i] : n[i])
                : "?";
 }
 inline const char* y_cfg_name(int i, int kind = 0) {
     static const char* n[kNumYCfg] = {"TX64xTY64", "TX64xTY32", "TX64xTY64/min12", "TX64xTY64/min16",
                                       "TX128xTY32/min5", "TX32xTY64"};
     static const char* nb[kNumYCfg] = {"TX64xTY64", "TX64xTY32", "TX32xTY32", "TX32xTY64", "TX128xTY32", "TX64xTY16"};
-    return (i >= 0 && i < kNumYCfg) ? ((kind == 1 || kind == 4) ? nb[i] : n[i]) : "?";
+    static const char* ns[kNumYCfg] = {"TX64xTY64", "TX64xTY32/min5", "TX64xTY64/min12", "TX64xTY64/min10", "TX128xTY32",
+                                       "TX32xTY64"};
+    static const char* nt[kNumYCfg] = {"TX64xTY64", "TX64xTY32", "TX32xTY32", "TX32xTY64", "TX128xTY32", "TX64xTY16/min5"};
+    return (i >= 0 && i < kNumYCfg)
+               ? (kind == 5 ? nt[i] : kind == 6 ? ns[i] : (kind == 1 || kind == 4) ? nb[i] : n[i]) : "?";
 }
 
 }  // namespace vg

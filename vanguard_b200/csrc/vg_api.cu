@@ -123,7 +123,7 @@ struct vg_solver {
     long last_launches = 0;
     int xcfg = 0, ycfg = 0;   // launch configuration of each sweep (sweep_table.cuh)
     int cfl_sep = 0;          // schedule: 0 folds the next step's CFL maximum into the last sweep, 1 a separate pass
-    int yseg = 0;             // Y segments: 0 the shape's TY, 1 sized for whole waves (sweep_table.cuh)
+    int yseg = 1;             // Y segments: 0 the shape's TY, 1 sized for the device (sweep_table.cuh)
     // TMA tensor maps over buf[0] and buf[1] for the TMA-staged X sweep (device memory; null: none)
     CUtensorMap* d_tmaps = nullptr;
     int tmap_planes = 0;
