@@ -23,6 +23,13 @@
 // matches it; everything else (edge states, fluxes, the derivative formulas) uses reciprocals refined to full
 // double precision and FMA contraction, which moves the gradient by round-off only.
 //
+// What bounds the reverse step: FP64 chains at 4 blocks of 128 threads an SM (126 registers; 96 and 166 take the same time to
+// 2 %, 80 spill).  The exact quotients share their reciprocals (exact_div.cuh) without branches, a stage whose operands leave
+// the proven range going through the compiler's division again; only cells that may attain S form the exact wave speed; a
+// block takes consecutive tiles, so that the step constants come once per instance and the next tile's state and adjoint
+// input are copied to shared memory behind this tile's arithmetic.  2.2 M cells in 1024 instances, 60 steps, 12 checkpoints:
+// 21.8 -> 20.9 ms with the shared reciprocals, 19.3 ms with the runs of tiles here and in the forward step.
+//
 // Tiles: AP = 128 positions per block, AH = 5 halo cells each side, AP - 2 AH outputs.  Every contribution to
 // r-bar and gamma-bar is owned by exactly one tile (interfaces by their right cell, or the last cell at the right
 // end; ghost-cell edges by the instance's end cells), so the per-instance sums are deterministic.  Ghost cells
@@ -32,10 +39,12 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/vanguard_slic.h"
 #include "batch_internal.cuh"
+#include "exact_div.cuh"
 #include "physics_mixed.cuh"
 #include "vg_ops.h"
 
@@ -56,63 +65,41 @@ struct Gas {
 };
 
 // EulerStateVector::computeConservedVariableVector (Euler/eulerstatevector.cpp:78-91), operation for operation
-__device__ __forceinline__ void cons_exact(const double* W, const Gas& q, double* U) {
+template <class D>
+__device__ __forceinline__ void cons_by(const double* W, const Gas& q, double* U, D& dv) {
     const double rho = W[0], u = W[1], p = W[2];
-    const double e = xdiv(xadd(p, xmul(q.g, q.pinf)), xmul(xsub(q.g, 1.0), rho));
+    const double e = dv.by(xmul(xsub(q.g, 1.0), rho)).positive(xadd(p, xmul(q.g, q.pinf)));
     U[0] = rho;
     U[1] = xmul(rho, u);
     U[2] = xmul(rho, xadd(xmul(0.5, xmul(u, u)), e));
+}
+__device__ __noinline__ double cons_energy_ieee(double rho, double u, double p, double g, double pinf) {
+    IeeeDiv dv;
+    Gas q;
+    q.g = g;
+    q.pinf = pinf;
+    const double W[3] = {rho, u, p};
+    double U[3];
+    cons_by(W, q, U, dv);
+    return U[2];
+}
+__device__ __forceinline__ void cons_exact(const double* W, const Gas& q, double* U) {
+    SharedDiv dv;
+    cons_by(W, q, U, dv);
+    if (!dv.ok()) U[2] = cons_energy_ieee(W[0], W[1], W[2], q.g, q.pinf);
 }
 // |u| + c of Solvers::computeMaximumWaveSpeed (Solvers/solvers.cpp:259-276), operation for operation
 __device__ __forceinline__ double wave_exact(double rho, double u, double p, double g, double pinf) {
     return xadd(fabs(u), __dsqrt_rn(xdiv(xmul(g, xadd(p, pinf)), rho)));
 }
-
-// xi(r) of SlopeLimiters::computeSlopeLimiter (Solvers/slopelimiters.cpp:7-74) with the derivative of the branch
-// taken; the comparisons see the forward's operands bit for bit (std::min(a, b) = b < a ? b : a).
-__device__ __forceinline__ void limiter_d(double r, double w, int id, double& xi, double& dxi) {
-    const double xr = xdiv(2.0, xadd(1.0 - w, xmul(1.0 + w, r)));
-    const double dxr = -0.5 * (1.0 + w) * xr * xr;  // d(2 / den)/dr = -2 (1 + w) / den^2
-    xi = 0.0;
-    dxi = 0.0;
-    if (r < 0.0) return;
-    if (id == 0) {
-        if (r < 0.5) {
-            xi = xmul(2.0, r);
-            dxi = 2.0;
-        } else if (r < 1.0) {
-            xi = 1.0;
-        } else {
-            const bool t = xr < r;
-            const double m1 = t ? xr : r;
-            if (!(2.0 < m1)) {
-                xi = m1;
-                dxi = t ? dxr : 1.0;
-            } else {
-                xi = 2.0;
-            }
-        }
-    } else if (id == 1) {
-        const double a = xdiv(xmul(2.0, r), xadd(1.0, r));
-        if (xr < a) {
-            xi = xr;
-            dxi = dxr;
-        } else {
-            const double ip = rcp_nr2(1.0 + r);
-            xi = a;
-            dxi = 2.0 * ip * ip;
-        }
-    } else {
-        if (r < 1.0) {
-            xi = r;
-            dxi = 1.0;
-        } else if (xr < 1.0) {
-            xi = xr;
-            dxi = dxr;
-        } else {
-            xi = 1.0;
-        }
-    }
+// Whether |u| + c equals the instance's maximum S, without the quotient and the root for the cells that are clearly below:
+// an equal sum has c >= (S - |u|) - 2^-53 S to within roundings, and c^2 from the refined reciprocal is good to a few 2^-53
+// (an inaccurate one, of a density that is subnormal or past the reciprocal's range, is not above 1e-200).
+__device__ __forceinline__ bool attains(double rho, double u, double p, double g, double pinf, double S) {
+    const double c2 = xmul(xmul(g, xadd(p, pinf)), rcp_nr2(rho));
+    const double d = (S - fabs(u)) - 1e-14 * S;
+    if (c2 > 1e-200 && d > 0.0 && d * d > c2 * (1.0 + 1e-10)) return false;
+    return wave_exact(rho, u, p, g, pinf) == S;
 }
 
 struct K {
@@ -120,20 +107,110 @@ struct K {
     int limiter;
 };
 
-// One slope component (SlopeLimiters::computeSlopeVector, Solvers/slopelimiters.cpp:217-246) and its partial
+// xi(r) of SlopeLimiters::computeSlopeLimiter (Solvers/slopelimiters.cpp:7-74) with the derivative of the branch
+// taken; the comparisons see the forward's operands bit for bit (std::min(a, b) = b < a ? b : a).  Every quotient is formed
+// and the ones that the branch does not reach are not used; without bias both divisors are 1 + r.
+template <int ID, class D>
+__device__ __forceinline__ void limiter_d(double r, double w, double& xi, double& dxi) {
+    const double den = xadd(1.0 - w, xmul(1.0 + w, r));
+    double xr, a = 0.0, ip = 0.0;
+    if constexpr (std::is_same<D, SharedDiv>::value) {
+        const double y = SharedDiv::reciprocal(den);
+        xr = SharedDiv::quotient(2.0, den, y);
+        if constexpr (ID == 1) {
+            const double b = xadd(1.0, r);
+            ip = w == 0.0 ? y : SharedDiv::reciprocal(b);
+            a = SharedDiv::quotient(xmul(2.0, r), b, ip);
+        }
+    } else {
+        xr = xdiv(2.0, den);
+        if constexpr (ID == 1) {
+            a = xdiv(xmul(2.0, r), xadd(1.0, r));
+            ip = 1.0 / (1.0 + r);
+        }
+    }
+    const double dxr = -0.5 * (1.0 + w) * xr * xr;  // d(2 / den)/dr = -2 (1 + w) / den^2
+    if constexpr (ID == 0) {
+        const bool t = xr < r;
+        const double m1 = t ? xr : r;
+        const bool capped = 2.0 < m1;
+        xi = r < 0.5 ? xmul(2.0, r) : r < 1.0 ? 1.0 : capped ? 2.0 : m1;
+        dxi = r < 0.5 ? 2.0 : (r < 1.0 || capped) ? 0.0 : t ? dxr : 1.0;
+    } else if constexpr (ID == 1) {
+        const bool t = xr < a;
+        xi = t ? xr : a;
+        dxi = t ? dxr : 2.0 * ip * ip;
+    } else {
+        const bool t = xr < 1.0;
+        xi = r < 1.0 ? r : t ? xr : 1.0;
+        dxi = r < 1.0 ? 1.0 : t ? dxr : 0.0;
+    }
+    if (r < 0.0) xi = dxi = 0.0;
+}
+
+// The slope components (SlopeLimiters::computeSlopeVector, Solvers/slopelimiters.cpp:217-246) and their partial
 // derivatives with respect to delta- = u - uL and delta+ = uR - u.
-__device__ __forceinline__ double slope_d(double uL, double u, double uR, const K& k, double& sdm, double& sdp) {
-    const double dm = u - uL, dp = uR - u;
-    const bool nf = fabs(dm) < k.floor5, df = fabs(dp) < k.floor5;
-    const double num = nf ? k.floor5 : dm, den = df ? k.floor5 : dp;
-    const double r = xdiv(num, den);
-    double xi, dxi;
-    limiter_d(r, k.bias, k.limiter, xi, dxi);
-    const double base = k.cm * dm + k.cp * dp;
-    const double t = base * dxi * rcp_nr2(den);  // base * dxi * dr/dnum
-    sdm = k.cm * xi + (nf ? 0.0 : t);
-    sdp = k.cp * xi - (df ? 0.0 : t * r);  // dr/dden = -r / den
-    return base * xi;
+template <int ID, class D>
+__device__ __forceinline__ void slopes_of(const double* uL, const double* u, const double* uR, const K& k, double* s,
+                                          double* sdm, double* sdp, D& dv) {
+#pragma unroll
+    for (int v = 0; v < 3; v++) {
+        const double dm = u[v] - uL[v], dp = uR[v] - u[v];
+        const bool nf = fabs(dm) < k.floor5, df = fabs(dp) < k.floor5;
+        const double num = nf ? k.floor5 : dm, den = df ? k.floor5 : dp;
+        double r, iden, xi, dxi;
+        if constexpr (std::is_same<D, SharedDiv>::value) {
+            dv.note_below(dm);
+            dv.note_below(dp);
+            iden = SharedDiv::reciprocal(den);
+            r = SharedDiv::quotient(num, den, iden);
+        } else {
+            iden = 1.0 / den;
+            r = xdiv(num, den);
+        }
+        limiter_d<ID, D>(r, k.bias, xi, dxi);
+        const double base = k.cm * dm + k.cp * dp;
+        const double t = base * dxi * iden;  // base * dxi * dr/dnum
+        sdm[v] = k.cm * xi + (nf ? 0.0 : t);
+        sdp[v] = k.cp * xi - (df ? 0.0 : t * r);  // dr/dden = -r / den
+        s[v] = base * xi;
+    }
+}
+template <class D>
+__device__ __forceinline__ void slopes_by(const double* uL, const double* u, const double* uR, const K& k, double* s,
+                                          double* sdm, double* sdp, D& dv) {
+    if (k.limiter == 0) slopes_of<0>(uL, u, uR, k, s, sdm, sdp, dv);
+    else if (k.limiter == 1) slopes_of<1>(uL, u, uR, k, s, sdm, sdp, dv);
+    else slopes_of<2>(uL, u, uR, k, s, sdm, sdp, dv);
+}
+__device__ __noinline__ void slopes_ieee(const double* in, const K* k, double* out) {
+    IeeeDiv dv;
+    slopes_by(in, in + 3, in + 6, *k, out, out + 3, out + 6, dv);
+}
+// The shared-reciprocal form, and again with the compiler's division where an operand left the proven range (or the bias
+// is one that the branch-free limiter does not cover).
+__device__ __forceinline__ void slopes_d(const double* uL, const double* u, const double* uR, const K& k, double* s,
+                                         double* sdm, double* sdp) {
+    SharedDiv dv;
+    const bool shared = fabs(k.bias) <= 1.0;
+    if (shared) slopes_by(uL, u, uR, k, s, sdm, sdp, dv);
+    if (!shared || !dv.ok()) {
+        double in[9], o[9];
+        K kc = k;
+#pragma unroll
+        for (int v = 0; v < 3; v++) {
+            in[v] = uL[v];
+            in[3 + v] = u[v];
+            in[6 + v] = uR[v];
+        }
+        slopes_ieee(in, &kc, o);
+#pragma unroll
+        for (int v = 0; v < 3; v++) {
+            s[v] = o[v];
+            sdm[v] = o[3 + v];
+            sdp[v] = o[6 + v];
+        }
+    }
 }
 
 // x flux of a conserved state with 1/rho kept for the vector-Jacobian product
@@ -190,7 +267,8 @@ __global__ void __launch_bounds__(AP, 4) adjoint_step_kernel(AdjArgs a) {
     // stage-aliased shared arrays: Us -> UL, Ea -> AB, Eb -> BB, Fs -> US
     __shared__ double S0[3][AP], S1[3][AP], S2[3][AP], S3[3][AP], MU[3][AP], UR[3][AP];
     __shared__ double red[2][AP / 32];
-    __shared__ double tile_k[4];  // dt/dx, dx/dt, 1/(gamma - 1) of the tile's instance, formed by one thread
+    __shared__ double tile_k[4];          // dt/dx, dx/dt, 1/(gamma - 1) of the instance, formed by one thread
+    __shared__ double Wn[3][AP], Ln[3][AP];  // the coming tile's state and adjoint input, a thread's own slots
     auto& Us = S0;
     auto& UL = S0;
     auto& Ea = S1;
@@ -200,50 +278,67 @@ __global__ void __launch_bounds__(AP, 4) adjoint_step_kernel(AdjArgs a) {
     auto& Fs = S3;
     auto& US = S3;
     const int p = threadIdx.x;
-    for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
-        const Tile tile = a.tiles[t];
-        const int k = tile.inst, n = a.ncell[k], s0 = tile.s0;
-        const long base = a.offset[k];
+    const int t0 = (int)((long)blockIdx.x * a.ntiles / gridDim.x);
+    const int t1 = (int)((blockIdx.x + 1L) * a.ntiles / gridDim.x);
+    if (t0 >= t1) return;
+    auto prefetch = [&](const Tile& tile) {
+        const long i = tile.base + ghost_index(tile.s0 - AH + p, tile.len, 0);
+        for (int v = 0; v < 3; v++) {
+            copy_async8(&Wn[v][p], a.W + v * a.plane + i);
+            copy_async8(&Ln[v][p], a.lam_in + v * a.plane + i);
+        }
+    };
+    K kc;
+    kc.cm = 0.5 * (1.0 + a.bias);
+    kc.cp = 0.5 * (1.0 - a.bias);
+    kc.bias = a.bias;
+    kc.floor5 = a.floor5;
+    kc.limiter = a.limiter;
+    Gas q{};
+    double Sk = 0.0;
+    int k = -1;
+    Tile next = a.tiles[t0];
+    prefetch(next);
+    for (int t = t0; t < t1; t++) {
+        const Tile tile = next;
+        if (t + 1 < t1) next = a.tiles[t + 1];
+        const int n = tile.len, s0 = tile.s0;
+        const long base = tile.base;
         const int c = s0 - AH + p;  // cell of this position (may be a ghost or beyond)
         const bool real = c >= 0 && c < n;
         const bool out = p >= AH && p < AP - AH && real;
         const bool owns_first = s0 == 0;                          // tile owning cell 0
         const bool owns_last = s0 <= n - 1 && n - 1 < s0 + AOUT;  // tile owning cell n-1
-        const double dxk = a.dx[k];
-        const double Sk = __longlong_as_double((long long)a.S[k]);
-        if (p == 0) {
-            const double dt = step_dt(a.cfl, dxk, Sk, a.step);
-            tile_k[0] = xdiv(dt, dxk);
-            tile_k[1] = dxk / dt;
-            tile_k[2] = 1.0 / (a.gam[2 * k] - 1.0);
+        if (tile.inst != k) {
+            k = tile.inst;
+            Sk = __longlong_as_double((long long)a.S[k]);
+            q.g = a.gam[2 * k];
+            q.pinf = a.gam[2 * k + 1];
+            q.gm1 = q.g - 1.0;
+            q.gpinf = q.g * q.pinf;
+            if (p == 0) {  // read after the first barrier below; the last instance's were read before the last tile's second
+                const double dt = step_dt(a.cfl, a.dx[k], Sk, a.step);
+                tile_k[0] = xdiv(dt, a.dx[k]);
+                tile_k[1] = a.dx[k] / dt;
+                tile_k[2] = 1.0 / (q.g - 1.0);
+            }
         }
-        K kc;
-        kc.cm = 0.5 * (1.0 + a.bias);
-        kc.cp = 0.5 * (1.0 - a.bias);
-        kc.bias = a.bias;
-        kc.floor5 = a.floor5;
-        kc.limiter = a.limiter;
-        Gas q;
-        q.g = a.gam[2 * k];
-        q.pinf = a.gam[2 * k + 1];
-        q.gm1 = q.g - 1.0;
-        q.gpinf = q.g * q.pinf;
-        // stage A: conserved vectors of every position (ghosts by the transmissive mirror); the adjoint input of
-        // the cells reverse 1 needs is loaded here so its latency hides behind stages B and C
+        // stage A: conserved vectors of every position (ghosts by the transmissive mirror)
         double W[3], lam[3] = {0.0, 0.0, 0.0};
         const bool upd = p >= 2 && p < AP - 2 && real;
         {
-            const int gi = ghost_index(c, n, 0);
-            for (int v = 0; v < 3; v++) W[v] = a.W[v * a.plane + base + gi];
+            copy_async_wait();
+            for (int v = 0; v < 3; v++) W[v] = Wn[v][p];
             if (upd)
-                for (int v = 0; v < 3; v++) lam[v] = a.lam_in[v * a.plane + base + c];
+                for (int v = 0; v < 3; v++) lam[v] = Ln[v][p];
             double U[3];
             cons_exact(W, q, U);
             for (int v = 0; v < 3; v++) Us[v][p] = U[v];
+            if (t + 1 < t1) prefetch(next);
         }
         // first cell of the instance attaining S (the CFL maximum's argmax)
         {
-            const unsigned hit = (out && wave_exact(W[0], W[1], W[2], q.g, q.pinf) == Sk) ? (unsigned)c : 0xffffffffu;
+            const unsigned hit = (out && attains(W[0], W[1], W[2], q.g, q.pinf, Sk)) ? (unsigned)c : 0xffffffffu;
             const unsigned m = __reduce_min_sync(0xffffffffu, hit);
             if ((p & 31) == 0 && m != 0xffffffffu) atomicMin(&a.arg[k], (int)m);
         }
@@ -255,11 +350,16 @@ __global__ void __launch_bounds__(AP, 4) adjoint_step_kernel(AdjArgs a) {
         // stage B: slopes (with their derivatives) and the evolved edge states of positions [1, AP-1)
         double xl[3], xr[3], dF[3], sdm[3], sdp[3], irl = 1.0, irr = 1.0;
         if (p >= 1 && p < AP - 1) {
+            double uL[3], u[3], uR[3], s[3];
             for (int v = 0; v < 3; v++) {
-                const double u = Us[v][p];
-                const double s = slope_d(Us[v][p - 1], u, Us[v][p + 1], kc, sdm[v], sdp[v]);
-                xl[v] = u - 0.5 * s;
-                xr[v] = u + 0.5 * s;
+                uL[v] = Us[v][p - 1];
+                u[v] = Us[v][p];
+                uR[v] = Us[v][p + 1];
+            }
+            slopes_d(uL, u, uR, kc, s, sdm, sdp);
+            for (int v = 0; v < 3; v++) {
+                xl[v] = u[v] - 0.5 * s[v];
+                xr[v] = u[v] + 0.5 * s[v];
             }
             double fl[3], fr[3];
             flux_a(xl, q, fl, irl);
@@ -421,7 +521,6 @@ __global__ void __launch_bounds__(AP, 4) adjoint_step_kernel(AdjArgs a) {
             a.tile_part[2 * t] = s1;
             a.tile_part[2 * t + 1] = s2;
         }
-        __syncthreads();
     }
 }
 
@@ -522,12 +621,10 @@ cudaError_t ensure_workspace(vg_batch* b, int checkpoints) {
     }
     if (b->lam[0]) return cudaSuccess;
     std::vector<vg::Tile> at;
-    std::vector<int> af(b->ninst), ac(b->ninst), order(b->ninst);
-    for (int k = 0; k < b->ninst; k++) order[k] = k;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return b->ncell[x] > b->ncell[y]; });
-    for (int k : order) {
+    std::vector<int> af(b->ninst), ac(b->ninst);
+    for (int k = 0; k < b->ninst; k++) {
         af[k] = (int)at.size();
-        for (int s0 = 0; s0 < b->ncell[k]; s0 += vg::AOUT) at.push_back({k, s0});
+        for (int s0 = 0; s0 < b->ncell[k]; s0 += vg::AOUT) at.push_back({b->offset[k], k, s0, b->ncell[k]});
         ac[k] = (int)at.size() - af[k];
     }
     b->natiles = (int)at.size();

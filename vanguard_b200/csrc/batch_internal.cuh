@@ -10,12 +10,20 @@
 
 namespace vg {
 
-constexpr int BP = 128;  // cells per tile segment of the forward step kernel (BP - 2 outputs)
+constexpr int BP = 128;  // cells per tile segment of the forward step kernel (BP - 4 outputs)
 
 struct Tile {
-    int inst;  // instance
-    int s0;    // first output cell within the instance
+    long base;  // first cell of the instance in the planes
+    int inst;   // instance
+    int s0;     // first output cell within the instance
+    int len;    // cells of the instance
 };
+
+// Eight bytes from global to shared memory behind this thread's back, and the wait for all of its copies.
+__device__ __forceinline__ void copy_async8(double* shared, const double* global) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(shared)), "l"(global) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 struct BatchArgs {
     const double* in;
@@ -74,7 +82,8 @@ struct vg_batch {
     int cur = 0;
     bool has_state = false;  // a successful vg_batch_upload has filled buf[0]
     bool nonfinite = false;  // a run since the upload flagged a non-finite or unphysical state
-    int grid = 0;
+    int grid = 0, grid_plain = 0;  // of the step kernel's two forms
+    bool plain = false;            // every instance has p_inf == 0
     cudaStream_t cap = nullptr;
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
