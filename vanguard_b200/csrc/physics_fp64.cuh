@@ -101,6 +101,11 @@ struct EulerF64 {
         double v = (NVEL == 2) ? W[2] : 0.0;
         return std_max(fabs(W[1]), fabs(v)) + c;
     }
+    // whether wave(W) is certainly below `floor`
+    __device__ static bool wave_below(const double* W, const P& q, int dims, double floor) {
+        const double v = (NVEL == 2 && dims != 1) ? W[2] : 0.0;
+        return certainly_below(floor, std_max(fabs(W[1]), fabs(v)), q.g * (W[IE] + q.pinf), W[0]);
+    }
     // EulerStateVector() (Euler/eulerstatevector.cpp:3-12)
     __device__ static void default_state(double* W) {
         for (int i = 0; i < NW; i++) W[i] = 0.0;
@@ -266,6 +271,12 @@ struct MHDF64 {
     __device__ static double wave(const double* W, const P& q, int dims) {
         if (dims == 1) return fabs(W[1]) + fabs(fast(W, q, W[IBX]));
         return std_max(fabs(W[1]), fabs(W[2])) + std_max(fabs(fast(W, q, W[IBX])), fabs(fast(W, q, W[IBY])));
+    }
+    // whether wave(W) is certainly below `floor`: a fast speed is at most the root of c^2 + |B|^2 / rho
+    __device__ static bool wave_below(const double* W, const P& q, int dims, double floor) {
+        const double x = q.g * (W[IP] + q.pinf), bz = FULL ? W[7] : 0.0;
+        return x >= 0.0 && certainly_below(floor, dims == 1 ? fabs(W[1]) : std_max(fabs(W[1]), fabs(W[2])),
+                                           x + (((W[IBX] * W[IBX]) + (W[IBY] * W[IBY])) + (bz * bz)), W[0]);
     }
     // MHDStateVector() (MHD/mhdstatevector.cpp:3-16)
     __device__ static void default_state(double* W) {

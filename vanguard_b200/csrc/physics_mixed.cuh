@@ -133,6 +133,10 @@ struct EulerMixed {
         double v = (NVEL == 2) ? W[2] : 0.0;
         return fmax(fabs(W[1]), fabs(v)) + c;
     }
+    __device__ static bool wave_below(const double* W, const P& q, int dims, double floor) {
+        const double v = (NVEL == 2 && dims != 1) ? W[2] : 0.0;
+        return certainly_below(floor, dims == 1 ? fabs(W[1]) : fmax(fabs(W[1]), fabs(v)), q.g * (W[IE] + q.pinf), W[0]);
+    }
     __device__ static void default_state(double* W) {
         for (int i = 0; i < NW; i++) W[i] = 0.0;
         W[0] = 1.0;
@@ -300,6 +304,11 @@ struct MHDMixed {
     __device__ static double wave(const double* W, const P& q, int dims) {
         if (dims == 1) return fabs(W[1]) + fast(W, q, W[IBX]);
         return fmax(fabs(W[1]), fabs(W[2])) + fmax(fast(W, q, W[IBX]), fast(W, q, W[IBY]));
+    }
+    __device__ static bool wave_below(const double* W, const P& q, int dims, double floor) {
+        const double x = q.g * (W[IP] + q.pinf);
+        return x >= 0.0 && certainly_below(floor, dims == 1 ? fabs(W[1]) : fmax(fabs(W[1]), fabs(W[2])),
+                                           x + sq3(W[IBX], W[IBY], FULL ? W[7] : 0.0), W[0]);
     }
     __device__ static void default_state(double* W) {
         for (int i = 0; i < NW; i++) W[i] = 0.0;

@@ -211,6 +211,7 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_mixed_kernel(SweepArgs a
     __shared__ double Us[NU][LPB][P + 2];
     __shared__ R Es[NU][LPB][P];
     __shared__ double Fs[NU][LPB][P];  // interface fluxes, widened once to FP64 for the update
+    __shared__ double wave_floor;
 
     const int p = threadIdx.x % P, l = threadIdx.x / P;
     const int row = blockIdx.y * LPB + l;
@@ -230,6 +231,8 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_mixed_kernel(SweepArgs a
     const MixedConst k = mixed_const(a, ts);
     const typename M::P q = M::params(a.params, a.ctrl ? a.ctrl->ch : a.ch_host);
 
+    const bool bounded = wave_bounded<M>(a);
+    const double so_far = wave_so_far(a, bounded);
     auto conserve = [&](int slot) {
         int c = ghost_index(s0 - 2 + slot, len, a.periodic);
         double W[NW], U[NU];
@@ -242,6 +245,7 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_mixed_kernel(SweepArgs a
     conserve(p + 1);
     if (p == 0) conserve(0);
     if (p == P - 1) conserve(P + 1);
+    if (threadIdx.x == 0) wave_floor = so_far;
     __syncthreads();
 
     R ub[NU];
@@ -282,12 +286,9 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_mixed_kernel(SweepArgs a
 #pragma unroll
         for (int v = 0; v < NW; v++) a.out[v * a.plane + rowbase + cell] = W[v];
         if (bad_state_mixed<M>(W, q)) atomicOr(a.err, ERR_STATE);
-        if (a.accumulate_wave) {
-            double s = M::wave(W, q, a.dims);
-            if (s > wave) wave = s;
-        }
+        if (a.accumulate_wave) raise_wave<M>(W, q, a.dims, wave_floor, wave);
     }
-    if (a.accumulate_wave) block_max_to<NT>(wave, a.wave_acc);
+    if (a.accumulate_wave) block_max_to<NT>(wave, a.wave_acc, bounded);
     if (a.advance_time && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         a.ctrl->t += a.ctrl->dt;
         a.ctrl->it += 1;
@@ -468,6 +469,7 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_pair_kernel(SweepArgs a)
     __shared__ double2 Us[NU][LPB][P + 2];
     __shared__ float2 Es[NU][LPB][P];
     __shared__ double2 Fs[NU][LPB][P];  // interface fluxes, widened once to FP64 for the update
+    __shared__ double wave_floor;
 
     const int p = threadIdx.x % P, l = threadIdx.x / P;
     const int row0 = (blockIdx.y * LPB + l) * 2;
@@ -489,6 +491,8 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_pair_kernel(SweepArgs a)
     const MixedConst k = mixed_const(a, ts);
     const typename M::P q = M::params(a.params, a.ctrl ? a.ctrl->ch : a.ch_host);
 
+    const bool bounded = wave_bounded<M>(a);
+    const double so_far = wave_so_far(a, bounded);
     auto conserve = [&](int slot) {
         int c = ghost_index(s0 - 2 + slot, len, a.periodic);
         double W0[NW], W1[NW], U0[NU], U1[NU];
@@ -505,6 +509,7 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_pair_kernel(SweepArgs a)
     conserve(p + 1);
     if (p == 0) conserve(0);
     if (p == P - 1) conserve(P + 1);
+    if (threadIdx.x == 0) wave_floor = so_far;
     __syncthreads();
 
     f2 ub[NU];
@@ -565,13 +570,10 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_pair_kernel(SweepArgs a)
 #pragma unroll
             for (int v = 0; v < NW; v++) a.out[v * a.plane + base[h] + cell] = W[v];
             if (bad_state_mixed<M>(W, q)) atomicOr(a.err, ERR_STATE);
-            if (a.accumulate_wave) {
-                double s = M::wave(W, q, a.dims);
-                if (s > wave) wave = s;
-            }
+            if (a.accumulate_wave) raise_wave<M>(W, q, a.dims, wave_floor, wave);
         }
     }
-    if (a.accumulate_wave) block_max_to<NT>(wave, a.wave_acc);
+    if (a.accumulate_wave) block_max_to<NT>(wave, a.wave_acc, bounded);
     if (a.advance_time && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         a.ctrl->t += a.ctrl->dt;
         a.ctrl->it += 1;

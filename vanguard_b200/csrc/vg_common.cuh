@@ -112,9 +112,17 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* addr, doub
     atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }
 
-// Block-wide max of non-negative doubles into *acc; call from all threads of the block.
+// Whether m + c is certainly below `floor` for a speed c with c^2 <= x / rho: without its quotient and roots, whose roundings
+// (and those of the sum) the margins cover.  False where an operand is a NaN, negative or far out of range.
+__device__ __forceinline__ bool certainly_below(double floor, double m, double x, double rho) {
+    const double d = floor * (1.0 - 1e-14) - m;
+    return d > 0.0 && d < 1e150 && rho > 0.0 && x >= 0.0 && (d * d) * rho > x * (1.0 + 1e-10) + 1e-290;
+}
+
+// Block-wide max of non-negative doubles into *acc; call from all threads of the block.  seldom: most blocks have none.
 template <int NT>
-__device__ __forceinline__ void block_max_to(double v, unsigned long long* acc) {
+__device__ __forceinline__ void block_max_to(double v, unsigned long long* acc, bool seldom = false) {
+    if (seldom && !__syncthreads_or(v > 0.0)) return;
     __shared__ double red[32];
     const unsigned full = 0xffffffffu;
 #pragma unroll
