@@ -26,9 +26,11 @@
 // What bounds the reverse step: FP64 chains at 4 blocks of 128 threads an SM (126 registers; 96 and 166 take the same time to
 // 2 %, 80 spill).  The exact quotients share their reciprocals (exact_div.cuh) without branches, a stage whose operands leave
 // the proven range going through the compiler's division again; only cells that may attain S form the exact wave speed; a
-// block takes consecutive tiles, so that the step constants come once per instance and the next tile's state and adjoint
-// input are copied to shared memory behind this tile's arithmetic.  2.2 M cells in 1024 instances, 60 steps, 12 checkpoints:
-// 21.8 -> 20.9 ms with the shared reciprocals, 19.3 ms with the runs of tiles here and in the forward step.
+// block takes consecutive tiles, so that the step constants come once per instance and the next tile's state is copied to
+// shared memory behind this tile's arithmetic.  The adjoint input is loaded where the tile begins: nothing waits for it before
+// the fluxes are done, and staging it as well made every tile wait for both (574 tiles, one a block: 8.5 us a step staged,
+// 8.1 loaded; 2672 tiles: 25.4 and 24.8).  2.2 M cells in 1024 instances, 60 steps, 12 checkpoints: 21.8 -> 20.9 ms with the
+// shared reciprocals, 19.3 ms with the runs of tiles here and in the forward step, 19.0 ms with their longer runs first.
 //
 // Tiles: AP = 128 positions per block, AH = 5 halo cells each side, AP - 2 AH outputs.  Every contribution to
 // r-bar and gamma-bar is owned by exactly one tile (interfaces by their right cell, or the last cell at the right
@@ -268,7 +270,7 @@ __global__ void __launch_bounds__(AP, 4) adjoint_step_kernel(AdjArgs a) {
     __shared__ double S0[3][AP], S1[3][AP], S2[3][AP], S3[3][AP], MU[3][AP], UR[3][AP];
     __shared__ double red[2][AP / 32];
     __shared__ double tile_k[4];          // dt/dx, dx/dt, 1/(gamma - 1) of the instance, formed by one thread
-    __shared__ double Wn[3][AP], Ln[3][AP];  // the coming tile's state and adjoint input, a thread's own slots
+    __shared__ double Wn[3][AP];          // the coming tile's state, a thread's own slots
     auto& Us = S0;
     auto& UL = S0;
     auto& Ea = S1;
@@ -278,15 +280,11 @@ __global__ void __launch_bounds__(AP, 4) adjoint_step_kernel(AdjArgs a) {
     auto& Fs = S3;
     auto& US = S3;
     const int p = threadIdx.x;
-    const int t0 = (int)((long)blockIdx.x * a.ntiles / gridDim.x);
-    const int t1 = (int)((blockIdx.x + 1L) * a.ntiles / gridDim.x);
+    const int t0 = first_tile(blockIdx.x, a.ntiles, gridDim.x), t1 = first_tile(blockIdx.x + 1, a.ntiles, gridDim.x);
     if (t0 >= t1) return;
     auto prefetch = [&](const Tile& tile) {
         const long i = tile.base + ghost_index(tile.s0 - AH + p, tile.len, 0);
-        for (int v = 0; v < 3; v++) {
-            copy_async8(&Wn[v][p], a.W + v * a.plane + i);
-            copy_async8(&Ln[v][p], a.lam_in + v * a.plane + i);
-        }
+        for (int v = 0; v < 3; v++) copy_async8(&Wn[v][p], a.W + v * a.plane + i);
     };
     K kc;
     kc.cm = 0.5 * (1.0 + a.bias);
@@ -330,7 +328,7 @@ __global__ void __launch_bounds__(AP, 4) adjoint_step_kernel(AdjArgs a) {
             copy_async_wait();
             for (int v = 0; v < 3; v++) W[v] = Wn[v][p];
             if (upd)
-                for (int v = 0; v < 3; v++) lam[v] = Ln[v][p];
+                for (int v = 0; v < 3; v++) lam[v] = a.lam_in[v * a.plane + base + c];
             double U[3];
             cons_exact(W, q, U);
             for (int v = 0; v < 3; v++) Us[v][p] = U[v];

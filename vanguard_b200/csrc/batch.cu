@@ -2,8 +2,8 @@
 //
 // Instances k = 0..K-1 have n_k cells (any sizes), their own gamma / p_inf and cell width dx_k, and are
 // concatenated into structure-of-arrays planes (rho, u, p) with a cell-offset table.  The work is cut into
-// tiles of BP - 4 consecutive cells of one instance; the blocks of a persistent grid share the tile table in equal runs, no
-// tile straddles two instances, and the transmissive ghosts of each instance are synthesised by the loader exactly as
+// tiles of BP - 4 consecutive cells of one instance; the blocks of a persistent grid share the tile table in runs of equal
+// length, no tile straddles two instances, and the transmissive ghosts of each instance are synthesised by the loader exactly as
 // Solvers::insertBoundaryCells builds them (Solvers/solvers.cpp:7-32).  Every instance takes its own time step
 // dt_k = CFL * dx_k / S_k (x0.2 for the first six steps, Solvers/solvers.cpp:437-452) from its own maximum wave
 // speed S_k, kept on the device in a three-slot ring: step s reads slot s % 3, accumulates the next maximum into
@@ -68,8 +68,11 @@ __device__ __forceinline__ double warp_max_nonneg(double w) {
 // pipe 49 % busy, barrier and long-scoreboard stalls 4.8 of 12 warps an issue).  So a block takes consecutive tiles, whose
 // instance changes seldom: the step constants and the flush of the running maximum come once per instance, and the next tile's
 // state is on its way to shared memory (each thread copies what it will read itself) during this tile's arithmetic.
-// Measured at 8.6 M cells in 4096 instances: 0.385 -> 0.340 ms a step (the form without p_inf and bias alone 0.378); 64, 72
-// and 80 registers (5 to 8 blocks an SM) take the same time as the uncapped 96.
+// The runs that are a tile longer are the first blocks', which the SMs hold evenly: at equal distances over the grid they met on
+// the same SMs (a distance times a number near a divisor of 148), and a batch of 1000 tiles took 0.73 ms for 60 steps against
+// 0.63 with every gridDim-th tile and 0.61 now.
+// 8.6 M cells in 4096 instances, 60 steps: 25.7 -> 19.7 ms (the form without p_inf and bias alone 25.2).  64, 72 and 80 registers
+// (5 to 8 blocks an SM) take the uncapped 96's time to 2 %, there and over 300 to 6000 tiles.
 template <class M>
 __global__ void __launch_bounds__(BP) batch_step_kernel(BatchArgs a) {
     constexpr int NU = M::NU, NW = M::NW;
@@ -82,8 +85,7 @@ __global__ void __launch_bounds__(BP) batch_step_kernel(BatchArgs a) {
     const int s = *a.step;
     const bool active = s < a.max_steps;
     const int slot_next = ((s + 1) % 3) * a.ninst;
-    const int t0 = (int)((long)blockIdx.x * a.ntiles / gridDim.x);
-    const int t1 = (int)((blockIdx.x + 1L) * a.ntiles / gridDim.x);
+    const int t0 = first_tile(blockIdx.x, a.ntiles, gridDim.x), t1 = first_tile(blockIdx.x + 1, a.ntiles, gridDim.x);
 
     auto prefetch = [&](const Tile& tile) {
         const long i = tile.base + ghost_index(tile.s0 - 2 + p, tile.len, 0);

@@ -19,6 +19,12 @@ struct Tile {
     int len;    // cells of the instance
 };
 
+// First of the consecutive tiles that a block takes: runs of equal length, the first blocks' one tile longer.
+__device__ __forceinline__ int first_tile(int block, int ntiles, int blocks) {
+    const int n = ntiles / blocks;
+    return block * n + min(block, ntiles - n * blocks);
+}
+
 // Eight bytes from global to shared memory behind this thread's back, and the wait for all of its copies.
 __device__ __forceinline__ void copy_async8(double* shared, const double* global) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(shared)), "l"(global) : "memory");
