@@ -32,13 +32,8 @@ template <class M, int AXIS, class D>
 __device__ __forceinline__ void frac_evolve_u(double c, const double* uL, double* uM, const double* uR, const SweepConst& k,
                                               const typename M::P& q, D& dv) {
     constexpr int NU = M::NU;
-    double s[NU], xl[NU], xr[NU], fl[NU], fr[NU];
-    slopes_by<NU, plain_set<M>::value>(uL, uM, uR, k, s, dv);
-#pragma unroll
-    for (int i = 0; i < NU; i++) {
-        xl[i] = uM[i] - (0.5 * s[i]);
-        xr[i] = uM[i] + (0.5 * s[i]);
-    }
+    double xl[NU], xr[NU], fl[NU], fr[NU];
+    edge_values<NU, plain_set<M>::value, false>(uL, uM, uR, k, xl, xr, dv);
     flux_by<M, AXIS>(xl, q, fl, dv);
     flux_by<M, AXIS>(xr, q, fr, dv);
 #pragma unroll

@@ -121,32 +121,56 @@ __device__ __forceinline__ double floored(double d, double floor5) {
     return m < (unsigned long long)__double_as_longlong(floor5) ? floor5 : d;
 }
 
-// SlopeLimiters::computeSlopeVector (Solvers/slopelimiters.cpp:217-246) of n components.  The limiter is chosen outside
-// the loop, so that the components' chains of divisions overlap.
-template <int ID, int N, bool UNBIASED, class D>
+// Edge values u -+ s / 2 of N components, s of SlopeLimiters::computeSlopeVector (Solvers/slopelimiters.cpp:217-246).
+// With shared reciprocals the limiter is chosen outside the loop, so that the components' chains of divisions overlap.
+template <int ID, int N, bool UNBIASED>
 __device__ __forceinline__ void slopes_of(const double* uL, const double* u, const double* uR, const SweepConst& k,
-                                          double* s, D& dv) {
+                                          double* s, SharedDiv& dv) {
 #pragma unroll
     for (int i = 0; i < N; i++) {
         const double dm = u[i] - uL[i], dp = uR[i] - u[i];
         const double num = floored(dm, k.floor5), den = floored(dp, k.floor5);
-        double phi;
-        if constexpr (std::is_same<D, SharedDiv>::value) {
-            dv.note_below(dm);
-            dv.note_below(dp);
-            phi = limiter_shared<ID, UNBIASED>(SharedDiv::known(num, den), k.bias);
-        } else {
-            phi = limiter_f64(num / den, k.bias, ID);
-        }
-        s[i] = ((k.cm * dm) + (k.cp * dp)) * phi;
+        dv.note_below(dm);
+        dv.note_below(dp);
+        s[i] = ((k.cm * dm) + (k.cp * dp)) * limiter_shared<ID, UNBIASED>(SharedDiv::known(num, den), k.bias);
     }
 }
-template <int N, bool UNBIASED, class D>
-__device__ __forceinline__ void slopes_by(const double* uL, const double* u, const double* uR, const SweepConst& k,
-                                          double* s, D& dv) {
+template <int N, bool UNBIASED, bool>
+__device__ __forceinline__ void edge_values(const double* uL, const double* u, const double* uR, const SweepConst& k,
+                                            double* xl, double* xr, SharedDiv& dv) {
+    double s[N];
     if (k.limiter == 0) slopes_of<0, N, UNBIASED>(uL, u, uR, k, s, dv);
     else if (k.limiter == 1) slopes_of<1, N, UNBIASED>(uL, u, uR, k, s, dv);
     else slopes_of<2, N, UNBIASED>(uL, u, uR, k, s, dv);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        xl[i] = u[i] - (0.5 * s[i]);
+        xr[i] = u[i] + (0.5 * s[i]);
+    }
+}
+// With the compiler's division.
+template <int N>
+__device__ __forceinline__ void edge_values_ieee(const double* uL, const double* u, const double* uR, const SweepConst& k,
+                                                 int limiter, double* xl, double* xr) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const double dm = u[i] - uL[i], dp = uR[i] - u[i];
+        double s = (k.cm * dm) + (k.cp * dp);
+        double num = dm, den = dp;
+        if (fabs(num) < k.floor5) num = k.floor5;
+        if (fabs(den) < k.floor5) den = k.floor5;
+        s = s * limiter_f64(num / den, k.bias, limiter);
+        xl[i] = u[i] - (0.5 * s);
+        xr[i] = u[i] + (0.5 * s);
+    }
+}
+template <int N, bool UNBIASED, bool IN_LOOP>
+__device__ __forceinline__ void edge_values(const double* uL, const double* u, const double* uR, const SweepConst& k,
+                                            double* xl, double* xr, IeeeDiv&) {
+    if (IN_LOOP) edge_values_ieee<N>(uL, u, uR, k, k.limiter, xl, xr);
+    else if (k.limiter == 0) edge_values_ieee<N>(uL, u, uR, k, 0, xl, xr);
+    else if (k.limiter == 1) edge_values_ieee<N>(uL, u, uR, k, 1, xl, xr);
+    else edge_values_ieee<N>(uL, u, uR, k, 2, xl, xr);
 }
 // whether the branch-free limiter covers this bias
 __device__ __forceinline__ bool bias_shared(double w) { return fabs(w) <= 1.0; }
@@ -154,17 +178,13 @@ __device__ __forceinline__ bool bias_shared(double w) { return fabs(w) <= 1.0; }
 // Solvers::evolveStateByHalf{X,Y}TimeStep for both sides of one cell (Solvers/solvers.cpp:454-466,
 // :502-514, :550-565): returns the conserved vectors of the two evolved edge states after the reference's
 // primitive round trip (setConservedVariableVector then computeConservedVariableVector).
-template <class M, int AXIS, class D>
+template <class M, int AXIS, bool IN_LOOP, class D>
 __device__ __forceinline__ void evolve_edges_by(const double* uL, const double* u, const double* uR, const SweepConst& k,
-                                                const typename M::P& q, double* ua_left_side, double* ua_right_side, D& dv) {
+                                                const typename M::P& q, double* ua_left_side, double* ua_right_side, D& dv,
+                                                bool want_left = true, bool want_right = true) {
     constexpr int NU = M::NU;
-    double s[NU], xl[NU], xr[NU], fl[NU], fr[NU];
-    slopes_by<NU, plain_set<M>::value>(uL, u, uR, k, s, dv);
-#pragma unroll
-    for (int i = 0; i < NU; i++) {
-        xl[i] = u[i] - (0.5 * s[i]);
-        xr[i] = u[i] + (0.5 * s[i]);
-    }
+    double xl[NU], xr[NU], fl[NU], fr[NU];
+    edge_values<NU, plain_set<M>::value, IN_LOOP>(uL, u, uR, k, xl, xr, dv);
     flux_by<M, AXIS>(xl, q, fl, dv);
     flux_by<M, AXIS>(xr, q, fr, dv);
     double a[NU], b[NU];
@@ -175,10 +195,14 @@ __device__ __forceinline__ void evolve_edges_by(const double* uL, const double* 
         b[i] = xr[i] + ev;
     }
     double w[M::NW];
-    setcons_by<M>(a, q, w, dv);
-    cons_by<M>(w, q, ua_left_side, dv);
-    setcons_by<M>(b, q, w, dv);
-    cons_by<M>(w, q, ua_right_side, dv);
+    if (want_left) {
+        setcons_by<M>(a, q, w, dv);
+        cons_by<M>(w, q, ua_left_side, dv);
+    }
+    if (want_right) {
+        setcons_by<M>(b, q, w, dv);
+        cons_by<M>(w, q, ua_right_side, dv);
+    }
 }
 
 // FirstOrderSolver::compute{X,Y}FORCEFlux (Solvers/firstordersolver.cpp:173-230) on the conserved vectors
@@ -205,7 +229,7 @@ __device__ __forceinline__ void force_flux_by(const double* ua, const double* ub
 template <class M, int AXIS>
 __device__ __noinline__ void evolve_edges_ieee(const double* in, const SweepConst* k, const typename M::P* q, double* out) {
     IeeeDiv dv;
-    evolve_edges_by<M, AXIS>(in, in + M::NU, in + 2 * M::NU, *k, *q, out, out + M::NU, dv);
+    evolve_edges_by<M, AXIS, true>(in, in + M::NU, in + 2 * M::NU, *k, *q, out, out + M::NU, dv);
 }
 template <class M, int AXIS>
 __device__ __noinline__ void force_flux_ieee(const double* in, const SweepConst* k, const typename M::P* q, double* F) {
@@ -223,13 +247,28 @@ __device__ __noinline__ void setcons_ieee(const double* U, const typename M::P* 
     setcons_by<M>(U, *q, W, dv);
 }
 
-template <class M, int AXIS>
+// How a sweep with the compiler's division saves registers, in a shape that caps them (CAPPED) or not.  Measured on 2048^2 Euler
+// multiphysics (X with 80 registers | Y with 96, 45 rows | Y uncapped, 56 rows) and MHD intermediate (Y, 56 rows), ms:
+//   the limiter chosen outside the loop over the components   0.762 | 0.991 | 1.140    1.733
+//   chosen for each component (IN_LOOP)                        0.734 | 0.978 | 1.161    1.796
+//   outside, and each row fetched one step ahead (AHEAD)             | 1.023 | 1.095    1.803
+//   the same, and both edges formed where one is read (BOTH)   0.788 | 1.023 | 1.064    1.786
+// So short states (the first model) save all they can where registers are capped and nothing where they are not; longer ones
+// have no use for a cap, and gain from the limiter's place alone.
+template <class M, bool CAPPED>
+struct ieee_form {
+    static constexpr bool SHORT = M::NU <= 9;
+    static constexpr bool IN_LOOP = SHORT && CAPPED, AHEAD = SHORT && !CAPPED, BOTH = SHORT && !CAPPED;
+};
+
+template <class M, int AXIS, bool CAPPED = false>
 __device__ __forceinline__ void evolve_edges(const double* uL, const double* u, const double* uR, const SweepConst& k,
-                                             const typename M::P& q, double* ua_left_side, double* ua_right_side) {
+                                             const typename M::P& q, double* ua_left_side, double* ua_right_side,
+                                             bool want_left = true, bool want_right = true) {
     if constexpr (shared_div<M>::value) {
         SharedDiv dv;
         const bool shared = bias_shared(k.bias);
-        if (shared) evolve_edges_by<M, AXIS>(uL, u, uR, k, q, ua_left_side, ua_right_side, dv);
+        if (shared) evolve_edges_by<M, AXIS, false>(uL, u, uR, k, q, ua_left_side, ua_right_side, dv);
         if (!shared || !dv.ok()) {
             constexpr int NU = M::NU;
             double in[3 * NU], out[2 * NU];
@@ -249,8 +288,10 @@ __device__ __forceinline__ void evolve_edges(const double* uL, const double* u, 
             }
         }
     } else {
+        using F = ieee_form<M, CAPPED>;
         IeeeDiv dv;
-        evolve_edges_by<M, AXIS>(uL, u, uR, k, q, ua_left_side, ua_right_side, dv);
+        evolve_edges_by<M, AXIS, F::IN_LOOP>(uL, u, uR, k, q, ua_left_side, ua_right_side, dv, F::BOTH || want_left,
+                                             F::BOTH || want_right);
     }
 }
 
@@ -505,7 +546,7 @@ __global__ void __launch_bounds__(P* LPB, MINB) sweep_x_kernel(SweepArgs a) {
             u[v] = Us[v][l][p + 1];
             uR[v] = Us[v][l][p + 2];
         }
-        evolve_edges<M, 0>(uL, u, uR, k, q, ub, ua);
+        evolve_edges<M, 0, (MINB > 1)>(uL, u, uR, k, q, ub, ua, p >= 1, p <= P - 2);
 #pragma unroll
         for (int v = 0; v < NU; v++) Es[v][l][p] = ua[v];
     }
@@ -570,19 +611,24 @@ __global__ void __launch_bounds__(TX, MINB) sweep_y_kernel(SweepArgs a) {
         cons_of<M>(W, q, U);
     };
 
-    double um1[NU], u0[NU], up1[NU], ua_prev[NU], f_prev[NU], dummy[NU], next[NW];
+    constexpr bool CAPPED = MINB > 1;
+    constexpr bool AHEAD = shared_div<M>::value || ieee_form<M, CAPPED>::AHEAD;  // each row is fetched one step ahead of its use
+    double um1[NU], u0[NU], up1[NU], ua_prev[NU], f_prev[NU], dummy[NU], next[AHEAD ? NW : 1];
     double wave = 0.0;
-    auto fetch = [&](int r) { load_w<M>(a, (long)ghost_index(r, len, a.periodic) * a.pitch + c, next); };
+    auto fetch = [&](int r) {
+        if constexpr (AHEAD) load_w<M>(a, (long)ghost_index(r, len, a.periodic) * a.pitch + c, next);
+    };
     conserve(r0 - 2, up1);   // temporarily holds row r0-2
     conserve(r0 - 1, um1);
     conserve(r0, u0);
-    fetch(r0 + 1);  // one row ahead of its use
-    evolve_edges<M, 1>(up1, um1, u0, k, q, dummy, ua_prev);   // right edge of row r0-1
+    fetch(r0 + 1);
+    evolve_edges<M, 1, CAPPED>(up1, um1, u0, k, q, dummy, ua_prev, false, true);   // right edge of row r0-1
     for (int r = r0; r <= r1; r++) {
-        cons_of<M>(next, q, up1);
+        if constexpr (AHEAD) cons_of<M>(next, q, up1);
+        else conserve(r + 1, up1);
         fetch(r + 2);
         double ub[NU], ua_next[NU];
-        evolve_edges<M, 1>(um1, u0, up1, k, q, ub, ua_next);
+        evolve_edges<M, 1, CAPPED>(um1, u0, up1, k, q, ub, ua_next, true, r < r1);
         double F[NU];
         force_flux<M, 1>(ua_prev, ub, k, q, F);     // flux at r - 1/2
         if (r > r0 && col_ok) {                      // update row r-1 with fluxes at r-3/2 and r-1/2
