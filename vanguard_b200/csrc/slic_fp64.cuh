@@ -22,7 +22,6 @@ namespace fp64 {
 constexpr int MW_NT = 256;
 
 struct Fp64Kernels {
-    static constexpr double ROW_LATENCY = 1.4;  // see y_segment_rows
     template <class M, int P, int LPB, int MINB>
     static void x(dim3 grid, int nt, cudaStream_t st, const SweepArgs& a) {
         plain_form<M>::pick(a, [&](auto m) { sweep_x_kernel<decltype(m), P, LPB, MINB><<<grid, nt, 0, st>>>(a); });

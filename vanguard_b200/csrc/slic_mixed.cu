@@ -13,7 +13,6 @@ namespace {
 constexpr int MW_NT = 256;
 
 struct MixedKernels {
-    static constexpr double ROW_LATENCY = 4.0;  // see y_segment_rows
     template <class M, int P, int LPB, int MINB>
     static void x(dim3 grid, int nt, cudaStream_t st, const SweepArgs& a) {
         if constexpr (M::PAIR_X) {

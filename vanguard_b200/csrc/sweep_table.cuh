@@ -29,24 +29,28 @@ cudaError_t launch_x(const SweepArgs& a, cudaStream_t st) {
 }
 
 // Rows marched per Y-sweep block when segments are sized for the device: the segment length from 2 to 4 TY that minimises
-// the time of the grid in units of one warp's row.  A scheduler with w resident warps takes max(latency, w) such units for a
-// row of all of them (latency: one warp's row alone against its share of a busy pipe), a block starts its march with about
-// 2.3 rows, every full wave of resident blocks runs at the full w, and the last one at what its blocks give each SM.  Measured
-// on the exact form, whose one warp per scheduler takes 1.4 of its pipe time (130 x 97 Euler: 35 us a sweep with the shape's
-// 64 rows, 9 us with 2; 2048^2 MHD: 0.296 ms with 64 rows, 0.253 ms with 32); the mixed form has shorter rows to hide the
-// same latency with.  The results do not depend on the segmentation.  The autotuner times every shape both ways.
-inline int y_segment_rows(int ny, int xblocks, int tx, long slots, int sms, double latency, int ty0) {
+// the time of the grid in units of one warp's share of its pipes for a row.  A scheduler with w resident warps takes
+// max(3, w + 0.4) such units for a row of all of them: one or two warps wait for their own chains, and many still do not fill
+// the pipes.  A block starts its march with about two rows, every full wave of resident blocks runs at the full w, and the last
+// one at what its blocks give each SM.  The rule was fitted to sweeps of every model family at 130 x 97, 512^2, 1024^2 and
+// 2048^2 with 2 to 128 rows; its choices are within 1.07 of the best of them, 1.003 on average.  (w alone, with a latency of 1.4
+// for the exact form, let a chip three fifths full pass for a full one: 2048^2 Euler multiphysics, blocks of 128 at 96 registers,
+// 1.16 ms with its 76 rows against 0.96 with 45, and 1.09 of the best on average.)  130 x 97 Euler: 43 us a sweep with 32 rows,
+// 13.8 us with 2; 2048^2 MHD: 0.289 ms with 64 rows, 0.257 ms with 56.  The results do not depend on the segmentation.  The
+// autotuner times every shape both ways.
+inline int y_segment_rows(int ny, int xblocks, int tx, long slots, int sms, int ty0) {
     if (slots <= 0 || sms <= 0 || ny <= 0) return ty0;
     const double warps = tx / 32.0 / 4.0;  // of one block on each scheduler
-    const double full = std::max(latency, (double)(slots / sms) * warps);
+    auto row = [](double w) { return std::max(3.0, w + 0.4); };
+    const double full = row((double)(slots / sms) * warps);
     int best = ty0;
     double best_cost = 1e300;
     for (int ty = 2; ty <= 4 * ty0; ty++) {
         const long blocks = (long)xblocks * ((ny + ty - 1) / ty);
         const long waves = blocks / slots, rest = blocks % slots;
         double cost = (double)waves * full;
-        if (rest) cost += std::max(latency, (double)((rest + sms - 1) / sms) * warps);
-        cost *= ty + 2.3;
+        if (rest) cost += row((double)((rest + sms - 1) / sms) * warps);
+        cost *= ty + 2;
         if (cost < best_cost) {
             best_cost = cost;
             best = ty;
@@ -78,7 +82,7 @@ cudaError_t launch_y(const SweepArgs& a0, cudaStream_t st) {
         if (a0.nx <= 0) return cudaSuccess;  // a call that only looks the occupancy up (before a graph capture)
         SweepArgs a = a0;
         const int xblocks = (a.nx + TX - 1) / TX;
-        a.ty_rows = a.y_waves ? y_segment_rows(a.ny, xblocks, TX, slots, sms, K::ROW_LATENCY, TY) : TY;
+        a.ty_rows = a.y_waves ? y_segment_rows(a.ny, xblocks, TX, slots, sms, TY) : TY;
         dim3 grid(xblocks, (a.ny + a.ty_rows - 1) / a.ty_rows);
         K::template y<M, TX, TY, MINB>(grid, TX, st, a);
         return cudaGetLastError();
