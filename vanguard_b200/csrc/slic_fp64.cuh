@@ -34,7 +34,15 @@ struct Fp64Kernels {
     }
     template <class M, int TX, int TY, int MINB>
     static void y(dim3 grid, int nt, cudaStream_t st, const SweepArgs& a) {
-        plain_form<M>::pick(a, [&](auto m) { sweep_y_kernel<decltype(m), TX, TY, MINB><<<grid, nt, 0, st>>>(a); });
+        sweep_y_kernel<M, TX, TY, MINB><<<grid, nt, 0, st>>>(a);
+    }
+    template <class M, class F>
+    static void form(const SweepArgs& a, F f) {
+        plain_form<M>::pick(a, f);
+    }
+    template <class M, class F>
+    static void each_form(F f) {
+        plain_form<M>::each(f);
     }
 };
 

@@ -40,12 +40,16 @@ template <class M>
 struct plain_set<M, decltype((void)M::PLAIN_SET)> {
     static constexpr bool value = M::PLAIN_SET;
 };
-// f(M::Plain{}) where the model has that form and the launch's parameters allow it, f(M{}) otherwise
+// pick: f(M::Plain{}) where the model has that form and the launch's parameters allow it, f(M{}) otherwise; each: f of all forms
 template <class M, class = void>
 struct plain_form {
     template <class F>
     static auto pick(const SweepArgs&, F f) {
         return f(M{});
+    }
+    template <class F>
+    static void each(F f) {
+        f(M{});
     }
 };
 template <class M>
@@ -53,6 +57,11 @@ struct plain_form<M, std::enable_if_t<!plain_set<M>::value && plain_set<typename
     template <class F>
     static auto pick(const SweepArgs& a, F f) {
         return a.bias == 0.0 && M::plain(a.params) ? f(typename M::Plain{}) : f(M{});
+    }
+    template <class F>
+    static void each(F f) {
+        f(M{});
+        f(typename M::Plain{});
     }
 };
 

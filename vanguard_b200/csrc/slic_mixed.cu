@@ -37,6 +37,14 @@ struct MixedKernels {
         const int grid = (int)(tiles < resident ? tiles : resident);
         sweep_x_tma_kernel<M, P, MINB><<<grid, P, 0, st>>>(a);
     }
+    template <class M, class F>
+    static void form(const SweepArgs&, F f) {
+        f(M{});
+    }
+    template <class M, class F>
+    static void each_form(F f) {
+        f(M{});
+    }
     template <class M, int TX, int TY, int MINB>
     static int y_resident() {
         int b = 0;

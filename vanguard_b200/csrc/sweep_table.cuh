@@ -60,31 +60,49 @@ inline int y_segment_rows(int ny, int xblocks, int tx, long slots, int sms, int 
     return best;
 }
 
-// Y sweep: TX columns per block, rows marched per thread from y_segment_rows (TY its centre), MINB as above.
+// Resident blocks of a Y shape on the device and its SMs, looked up on first use (every thread stores the same).
+template <class K, class M, int TX, int TY, int MINB>
+long y_slots(int& sms) {
+    static std::atomic<long> cached{0};
+    static std::atomic<int> cached_sms{0};
+    long slots = cached.load(std::memory_order_acquire);
+    if (slots == 0) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        slots = (long)K::template y_resident<M, TX, TY, MINB>() * n;
+        if (slots <= 0) slots = -1;
+        cached_sms.store(n, std::memory_order_relaxed);
+        cached.store(slots, std::memory_order_release);
+    }
+    sms = cached_sms.load(std::memory_order_relaxed);
+    return slots;
+}
+
+// Y sweep: TX columns per block, rows marched per thread from y_segment_rows (TY its centre), MINB as above.  The segments are
+// sized for the form of the model that the launch takes: the plain Euler form has 164 registers where the general one has 190.
 template <class K, class M, int TX, int TY, int MINB>
 cudaError_t launch_y(const SweepArgs& a0, cudaStream_t st) {
     if constexpr (!M::HAS_Y) {
         return cudaErrorInvalidValue;
     } else {
-        static std::atomic<long> cached{0};  // resident blocks of this shape on the device (every thread stores the same)
-        static std::atomic<int> cached_sms{0};
-        long slots = cached.load(std::memory_order_acquire);
-        if (slots == 0) {
-            int dev = 0, n = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-            slots = (long)K::template y_resident<M, TX, TY, MINB>() * n;
-            if (slots <= 0) slots = -1;
-            cached_sms.store(n, std::memory_order_relaxed);
-            cached.store(slots, std::memory_order_release);
+        if (a0.nx <= 0) {  // a call that only looks the occupancy up (before a graph capture)
+            K::template each_form<M>([](auto m) {
+                int sms;
+                y_slots<K, decltype(m), TX, TY, MINB>(sms);
+            });
+            return cudaSuccess;
         }
-        const int sms = cached_sms.load(std::memory_order_relaxed);
-        if (a0.nx <= 0) return cudaSuccess;  // a call that only looks the occupancy up (before a graph capture)
-        SweepArgs a = a0;
-        const int xblocks = (a.nx + TX - 1) / TX;
-        a.ty_rows = a.y_waves ? y_segment_rows(a.ny, xblocks, TX, slots, sms, TY) : TY;
-        dim3 grid(xblocks, (a.ny + a.ty_rows - 1) / a.ty_rows);
-        K::template y<M, TX, TY, MINB>(grid, TX, st, a);
+        K::template form<M>(a0, [&](auto m) {
+            using F = decltype(m);
+            SweepArgs a = a0;
+            const int xblocks = (a.nx + TX - 1) / TX;
+            int sms;
+            const long slots = y_slots<K, F, TX, TY, MINB>(sms);
+            a.ty_rows = a.y_waves ? y_segment_rows(a.ny, xblocks, TX, slots, sms, TY) : TY;
+            dim3 grid(xblocks, (a.ny + a.ty_rows - 1) / a.ty_rows);
+            K::template y<F, TX, TY, MINB>(grid, TX, st, a);
+        });
         return cudaGetLastError();
     }
 }
