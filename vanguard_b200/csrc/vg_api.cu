@@ -984,8 +984,11 @@ vg_status vg_autotune(vg_solver* s, const vg_run_config* cfg, int reps, float* t
             b.accumulate_wave = sc == 0;
             SweepArgs m = base_args(s);
             m.in = a.out;
+            // the accumulator starts from zero in every repetition, as in a step: an X sweep that finds the maximum already there
+            // leaves out the exact speeds that a step's first wave of blocks has to form
             auto tail = [&]() {
-                cudaError_t e = xfn(b, st);
+                cudaError_t e = cudaMemsetAsync(&s->ctrl->smax_next, 0, sizeof(s->ctrl->smax_next), st);
+                if (e == cudaSuccess) e = xfn(b, st);
                 if (sc == 1 && e == cudaSuccess) e = s->ops->max_wave(m, st);
                 return e;
             };
