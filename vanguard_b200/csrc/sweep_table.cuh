@@ -149,6 +149,9 @@ constexpr int tile_kind() {
            : shared_sweeps<M>::value ? 6 : 0;
 }
 
+// Revision of the tables below, part of the key of saved tunings: raise it where an index comes to name another shape.
+constexpr int kSweepTables = 2;
+
 template <class K, class M, int KIND = tile_kind<M>()>
 struct SweepTable;
 

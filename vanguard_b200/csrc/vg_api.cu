@@ -190,8 +190,9 @@ void build_tmaps(vg_solver* s, int planes) {
     s->tmap_planes = planes;
 }
 
-// In-process cache of tuned launch configurations keyed by variant, precision, grid and SM count;
-// optionally persisted in the text file named by VG_TUNE_CACHE ("key xcfg ycfg" per line).
+// In-process cache of tuned launch configurations keyed by variant, precision, boundary, grid, SM count and shape table (its
+// kind and revision: the indices of another table name other shapes); optionally persisted in the text file named by
+// VG_TUNE_CACHE ("key xcfg ycfg schedule y-segments" per line).
 struct TuneEntry {
     std::string key;
     int xcfg, ycfg, sched, yseg;
@@ -203,8 +204,8 @@ std::string tune_key(const vg_solver* s) {
     int dev = s->d.device, sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     char buf[160];
-    std::snprintf(buf, sizeof(buf), "v%d_p%d_b%d_%dx%d_sm%d", s->variant, s->d.precision, s->d.boundary, s->d.nx,
-                  s->d.ny, sms);
+    std::snprintf(buf, sizeof(buf), "v%d_p%d_b%d_%dx%d_sm%d_k%dr%d", s->variant, s->d.precision, s->d.boundary, s->d.nx,
+                  s->d.ny, sms, s->ops->tile_kind, vg::kSweepTables);
     return buf;
 }
 
