@@ -43,3 +43,19 @@ def test_lines_of_another_table_are_tuned_again(tmp_path):
         cache.write_text(f"{stale} 3 2 1 0\n")
         _, lines = _apply(cache)
         assert [ln[0] for ln in lines] == [stale, key]
+
+
+def test_names_give_the_register_caps(gpu):
+    """Index 0 of the exact models' tables, whose caps differ by the length of the state."""
+    from vanguard_b200 import workloads as wl
+    names = []
+    for model, W, prm in ((gpu.EULER, wl.euler_quadrants_2d(40, 30, seed=1), wl.euler_params()),
+                          (gpu.EULER_REDUCED, wl.reduced_bubble_2d(40, 30), wl.reduced_params()),
+                          (gpu.MHD, wl.mhd_vortex_2d(40, 30, seed=1), wl.mhd_params())):
+        if model == gpu.MHD:
+            W[3] = 0.1  # all nine planes
+        with gpu.Solver(model, 40, 30, prm) as s:
+            s.upload(W)
+            s.set_launch_config(0, 0)
+            names.append(s.launch_config()[2:])
+    assert names == [("P128xL1/min7", "TX64xTY64/min8"), ("P128xL1/min7", "TX64xTY64"), ("P128xL1/min4", "TX64xTY64")]

@@ -128,7 +128,7 @@ struct pair_sweeps<M, decltype((void)M::PAIR_X)> {
 
 // The exact-form models with shared reciprocals (exact_div.cuh) have long independent chains that the compiler would overlap
 // with every register it can get; their own tables cap the registers where more resident warps pay more (kinds 5 and 6,
-// index 0 the default).
+// index 0 the default).  The caps of kinds 7 and 8, kind 6 of longer states, differ in those shapes alone.
 template <class M, class = void>
 struct shared_sweeps {
     static constexpr bool value = false;
@@ -146,7 +146,7 @@ struct shared_sweeps<M, decltype((void)M::SHARED_DIV)> {
 template <class M>
 constexpr int tile_kind() {
     return (M::NU > 21) ? 4 : (M::NU > 9) ? (shared_sweeps<M>::value ? 5 : 1) : pair_sweeps<M>::value ? (M::NW <= 4 ? 2 : 3)
-           : shared_sweeps<M>::value ? 6 : 0;
+           : shared_sweeps<M>::value ? (M::NU <= 4 ? 6 : M::NU <= 7 ? 7 : 8) : 0;
 }
 
 // Revision of the tables below, part of the key of saved tunings: raise it where an index comes to name another shape.
@@ -219,9 +219,8 @@ struct SweepTable<K, M, 3> {
 // registers) 0.648 | 0.266 | 0.335 | -, 5 (96) 0.689 | 0.264 | 0.332 | 0.403, 4 (128) 0.730 | 0.271 | 0.337 | 0.339, no cap 0.73 |
 // 0.38 | 0.45 | 0.36.  Y: 8 blocks of 64 (128 registers) 0.606 for Euler against 0.616 without a cap; the longer states lose
 // more to spills than the warps give (MHD7 0.291 against 0.253, two-material Euler 0.358 against 0.344).
-template <class K, class M>
-struct SweepTable<K, M, 6> {
-    static constexpr int XB = M::NU <= 7 ? 7 : 4, YB = M::NU <= 4 ? 8 : 1;
+template <class K, class M, int XB, int YB>
+struct SharedSweepTable {
     static constexpr SweepFn x[kNumXCfg] = {
         launch_x<K, M, 128, 1, XB>, launch_x<K, M, 64, 1, 9>, launch_x<K, M, 96, 1, 8>,
         launch_x<K, M, 128, 1, 5>, launch_x<K, M, 128, 1, 8>,
@@ -231,6 +230,13 @@ struct SweepTable<K, M, 6> {
         launch_y<K, M, 64, 64, 10>, launch_y<K, M, 128, 32, 1>, launch_y<K, M, 32, 64, YB>,
     };
 };
+
+template <class K, class M>
+struct SweepTable<K, M, 6> : SharedSweepTable<K, M, 7, 8> {};
+template <class K, class M>
+struct SweepTable<K, M, 7> : SharedSweepTable<K, M, 7, 1> {};
+template <class K, class M>
+struct SweepTable<K, M, 8> : SharedSweepTable<K, M, 4, 1> {};
 
 // X (1001x777 two-material MHD | 1024^2 HPR): 4 blocks of 96 (168 registers) 0.118 | 0.271, 5 of 64 (168) 0.119 | 0.291, no cap
 // 0.135 | 0.288.
@@ -248,26 +254,32 @@ struct SweepTable<K, M, 5> {
 
 // Names of the shapes of SweepTable<K, M, kind>.
 inline const char* x_cfg_name(int i, int kind = 0) {
-    static const char* n[kNumXCfg] = {"P128xL1", "P64xL2", "P192xL1", "P128xL1/min6", "P128xL1/min8"};
-    static const char* nb[kNumXCfg] = {"P64xL1", "P32xL2", "P96xL1", "P64xL1/min2", "P32xL1"};
-    static const char* np[kNumXCfg] = {"P128x2", "TMA P128x2/min7", "TMA P128x2/min8", "P128x2/min6", "P128x2/min8"};
-    static const char* nq[kNumXCfg] = {"P128x2", "P64xL2x2", "P128x2/min4", "P128x2/min6", "P128x2/min8"};
-    static const char* nw[kNumXCfg] = {"P32xL1", "P40xL1", "P48xL1", "P56xL1", "P32xL1/min2"};
-    static const char* ns[kNumXCfg] = {"P128xL1", "P64xL1/min9", "P96xL1/min8", "P128xL1/min5", "P128xL1/min8"};
-    static const char* nt[kNumXCfg] = {"P96xL1/min4", "P64xL1/min5", "P64xL1", "P32xL2/min5", "P32xL1"};
-    return (i >= 0 && i < kNumXCfg)
-               ? (kind == 5 ? nt[i] : kind == 6 ? ns[i] : kind == 1 ? nb[i] : kind == 2 ? np[i] : kind == 3 ? nq[i] : kind == 4 ? nw[i] : n[i])
-               : "?";
+    static const char* const n[][kNumXCfg] = {
+        {"P128xL1", "P64xL2", "P192xL1", "P128xL1/min6", "P128xL1/min8"},
+        {"P64xL1", "P32xL2", "P96xL1", "P64xL1/min2", "P32xL1"},
+        {"P128x2", "TMA P128x2/min7", "TMA P128x2/min8", "P128x2/min6", "P128x2/min8"},
+        {"P128x2", "P64xL2x2", "P128x2/min4", "P128x2/min6", "P128x2/min8"},
+        {"P32xL1", "P40xL1", "P48xL1", "P56xL1", "P32xL1/min2"},
+        {"P96xL1/min4", "P64xL1/min5", "P64xL1", "P32xL2/min5", "P32xL1"},
+        {"P128xL1/min7", "P64xL1/min9", "P96xL1/min8", "P128xL1/min5", "P128xL1/min8"},
+        {"P128xL1/min7", "P64xL1/min9", "P96xL1/min8", "P128xL1/min5", "P128xL1/min8"},
+        {"P128xL1/min4", "P64xL1/min9", "P96xL1/min8", "P128xL1/min5", "P128xL1/min8"},
+    };
+    return i >= 0 && i < kNumXCfg && kind >= 0 && kind < 9 ? n[kind][i] : "?";
 }
 inline const char* y_cfg_name(int i, int kind = 0) {
-    static const char* n[kNumYCfg] = {"TX64xTY64", "TX64xTY32", "TX64xTY64/min12", "TX64xTY64/min16",
-                                      "TX128xTY32/min5", "TX32xTY64"};
-    static const char* nb[kNumYCfg] = {"TX64xTY64", "TX64xTY32", "TX32xTY32", "TX32xTY64", "TX128xTY32", "TX64xTY16"};
-    static const char* ns[kNumYCfg] = {"TX64xTY64", "TX64xTY32/min5", "TX64xTY64/min12", "TX64xTY64/min10", "TX128xTY32",
-                                       "TX32xTY64"};
-    static const char* nt[kNumYCfg] = {"TX64xTY64", "TX64xTY32", "TX32xTY32", "TX32xTY64", "TX128xTY32", "TX64xTY16/min5"};
-    return (i >= 0 && i < kNumYCfg)
-               ? (kind == 5 ? nt[i] : kind == 6 ? ns[i] : (kind == 1 || kind == 4) ? nb[i] : n[i]) : "?";
+    static const char* const n[][kNumYCfg] = {
+        {"TX64xTY64", "TX64xTY32", "TX64xTY64/min12", "TX64xTY64/min16", "TX128xTY32/min5", "TX32xTY64"},
+        {"TX64xTY64", "TX64xTY32", "TX32xTY32", "TX32xTY64", "TX128xTY32", "TX64xTY16"},
+        {"TX64xTY64", "TX64xTY32", "TX64xTY64/min12", "TX64xTY64/min16", "TX128xTY32/min5", "TX32xTY64"},
+        {"TX64xTY64", "TX64xTY32", "TX64xTY64/min12", "TX64xTY64/min16", "TX128xTY32/min5", "TX32xTY64"},
+        {"TX64xTY64", "TX64xTY32", "TX32xTY32", "TX32xTY64", "TX128xTY32", "TX64xTY16"},
+        {"TX64xTY64", "TX64xTY32", "TX32xTY32", "TX32xTY64", "TX128xTY32", "TX64xTY16/min5"},
+        {"TX64xTY64/min8", "TX64xTY32/min5", "TX64xTY64/min12", "TX64xTY64/min10", "TX128xTY32", "TX32xTY64/min8"},
+        {"TX64xTY64", "TX64xTY32/min5", "TX64xTY64/min12", "TX64xTY64/min10", "TX128xTY32", "TX32xTY64"},
+        {"TX64xTY64", "TX64xTY32/min5", "TX64xTY64/min12", "TX64xTY64/min10", "TX128xTY32", "TX32xTY64"},
+    };
+    return i >= 0 && i < kNumYCfg && kind >= 0 && kind < 9 ? n[kind][i] : "?";
 }
 
 }  // namespace vg

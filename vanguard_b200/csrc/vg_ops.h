@@ -43,7 +43,7 @@ struct Ops {
     // One relaxation-source sub-cycle of length 0.5 dt / subcycles, a.in -> a.out, with a.aux as scratch
     // (kForcingLaunches kernels; null: model has no source).
     cudaError_t (*forcing)(const SweepArgs& a, int subcycles, cudaStream_t st);
-    int tile_kind;  // SweepTable kind: 0 default, 1 big models, 2 PAIR_X models (names of the launch configurations)
+    int tile_kind;  // SweepTable kind (names of the launch configurations, key of saved tunings)
     // First-order FORCE sweeps (FirstOrderSolver), null where the form has none.
     SweepFn x1 = nullptr;
     SweepFn y1 = nullptr;
