@@ -129,9 +129,14 @@ __device__ __forceinline__ void forcing_cell(const SweepArgs& a, int subcycles, 
     cons_by<M>(W, q, uM, dv);
     source_by<M>(uM, q, S, dv);
     for (int v = 0; v < NU; v++) kk(0, v) = dt * S[v];
+    // out of range already (mostly a heat flux that has decayed to nothing): the caller evaluates the cell again, and this pass
+    // leaves out its stages
+    int stages = 3;
+    if constexpr (std::is_same<D, SharedDiv>::value)
+        if (!dv.ok()) stages = 0;
     const double stage_frac[3] = {0.5, 0.5, 1.0};
 #pragma unroll 1
-    for (int s = 0; s < 3; s++) {
+    for (int s = 0; s < stages; s++) {
         double um[NU], wm[NW];
         for (int v = 0; v < NU; v++) um[v] = uM[v] + (s < 2 ? (0.5 * kk(s, v)) : kk(s, v));
         // set into a default-constructed state and converted back, here and after each predictor: the two conversions
