@@ -411,7 +411,6 @@ struct EulerReducedModel {
         W[4] = 1.0;
         W[5] = 1.0;
     }
-    // the smaller material density (bad-state check: both must stay positive) and the interface pressure
     // the same with the compiler's division
     __device__ static void cons(const double* W, const P& q, double* U) {
         IeeeDiv dv;
@@ -426,6 +425,7 @@ struct EulerReducedModel {
         IeeeDiv dv;
         flux<AXIS>(U, q, F, dv);
     }
+    // the smaller material density (bad-state check: both must stay positive) and the interface pressure
     __device__ static double density(const double* W) { return W[3] < W[4] ? W[3] : W[4]; }
     __device__ static double pressure(const double* W) { return W[5]; }
 };
@@ -681,7 +681,6 @@ struct MHDReducedModel {
         W[5] = 1.0;
         W[6] = 1.0;
     }
-    // the smaller material density (bad-state check) and the interface pressure
     // the same with the compiler's division
     __device__ static void cons(const double* W, const P& q, double* U) {
         IeeeDiv dv;
@@ -700,6 +699,7 @@ struct MHDReducedModel {
         IeeeDiv dv;
         source(U, q, S, dv);
     }
+    // the smaller material density (bad-state check) and the interface pressure
     __device__ static double density(const double* W) { return W[4] < W[5] ? W[4] : W[5]; }
     __device__ static double pressure(const double* W) { return W[6]; }
 };

@@ -942,7 +942,7 @@ vg_status vg_autotune(vg_solver* s, const vg_run_config* cfg, int reps, float* t
     int pick[2] = {0, 0}, pick_yseg = 0;
     for (int axis = 0; axis < s->dims; axis++) {
         int n = axis == 0 ? vg::kNumXCfg : vg::kNumYCfg;
-        // each Y shape is timed with its own segment length and with segments sized for whole waves
+        // each Y shape is timed with its own segment length and with segments sized for the device
         for (int c = 0; c < n * (axis == 0 ? 1 : 2); c++) {
             const int shape = c % n;
             const vg::SweepFn fn = axis == 0 ? s->ops->x[shape] : s->ops->y[shape];
