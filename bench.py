@@ -381,7 +381,7 @@ def run_cuda(args, world, rank, local):
                                + r["tuned"]["x"] + ")",
                      "algorithmic_bytes_per_launch": x_bytes, "peak_source": peak_kind,
                      "note": ("the exact FP64 form is bound by the FP64 pipe (correctly rounded divisions and square "
-                              "roots, no contraction), not by HBM: ncu shows the FP64 pipe 61 % busy and DRAM 10 % "
+                              "roots, no contraction), not by HBM: ncu shows the FP64 pipe 63 % busy and DRAM 15 % "
                               "(profiles/sweep_x_kernel_euler_fp64_2048.md); the mixed form's X sweep reaches 0.62 of "
                               "HBM (forms.mixed.x_sweep_hbm_frac)") if head == "fp64" else ""},
         "e2e": {"value": job_value(world, cells * args.steps, e2e_s), "unit": UNIT,
